@@ -74,8 +74,8 @@ BatchState &bstate() {
 }
 
 struct BatchPlan {
-    std::vector<DeviceScene> scenes;
-    std::vector<uint32_t> work_base, pixel_base;
+    std::vector<DeviceScene> scenes;                // in work order (work_order), not the caller's
+    std::vector<uint32_t> work_base, pixel_base;    // of scenes[k]; pixel_base is its place in the caller's order
     uint32_t spp = 0, max_bounces = 0;
     uint64_t pixels = 0, work = 0, key = 0;
 };
@@ -88,13 +88,40 @@ uint64_t fnv(uint64_t h, uint64_t v) {
     return h;
 }
 
+// Order of the scenes' work in a pass: by formula, the dearest step first, and
+// by falling iteration count within a formula.  Several scenes are in flight
+// at once (the persistent march holds about 136k rays, a scene of the
+// 64-scene workload has 65k a pass), and a warp's lanes are refilled from the
+// head of the queue at different times: in the caller's order a warp runs the
+// orbit loops of up to three formulas one after the other.  A path's result
+// does not depend on the order.
+uint64_t scene_work(const DeviceScene &S) { return uint64_t((S.width + 7u) / 8u) * ((S.height + 3u) / 4u) * 32u; }   // 8 x 4 tiles
+int step_cost(uint32_t kind) {
+    switch (kind) {
+        case KIND_BULB: return 0;
+        case KIND_HYBRID: return 1;
+        case KIND_BULB8: return 2;
+        case KIND_BOX: return 3;
+        default: return 4;
+    }
+}
+std::vector<size_t> work_order(const std::vector<DeviceScene> &scenes) {
+    std::vector<size_t> order(scenes.size());
+    for (size_t k = 0; k < order.size(); ++k) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+        const int ca = step_cost(scenes[a].kind), cb = step_cost(scenes[b].kind);
+        return ca != cb ? ca < cb : scenes[a].iterations > scenes[b].iterations;
+    });
+    return order;
+}
+
 bool make_plan(const FptRenderConfig *configs, const FptCudaSceneExt *exts, size_t count, BatchPlan &P, char *error,
                size_t error_len) {
     if (!configs || !exts || count == 0) { set_error(error, error_len, "a batch needs configs, extensions and count > 0"); return false; }
     if (count > 65535) { set_error(error, error_len, "a batch holds at most 65535 scenes"); return false; }
-    P.scenes.resize(count);
-    P.work_base.assign(count + 1, 0);
-    P.pixel_base.assign(count + 1, 0);
+    std::vector<DeviceScene> scenes(count);
+    std::vector<uint32_t> pixel_base(count + 1, 0);
+    uint64_t total_work = 0;
     uint64_t key = 1469598103934665603ull;
     for (size_t k = 0; k < count; ++k) {
         const FptRenderConfig &c = configs[k];
@@ -106,27 +133,35 @@ bool make_plan(const FptRenderConfig *configs, const FptCudaSceneExt *exts, size
         if (c.renderer_backend != FPT_RENDERER_SDF) { set_error(error, error_len, "scene %zu: batched scenes use the SDF renderer", k); return false; }
         FptRenderConfig h = c;
         if (!hydrate_hdri(h, error, error_len)) return false;
-        if (!compile_scene(h, &e, P.scenes[k], error, error_len)) return false;
-        const DeviceScene &S = P.scenes[k];
+        if (!compile_scene(h, &e, scenes[k], error, error_len)) return false;
+        const DeviceScene &S = scenes[k];
         if (k == 0) P.spp = S.samples;
         if (S.samples != P.spp || S.samples == 0) {
             set_error(error, error_len, "scene %zu: every scene of a batch takes the same sample count (> 0)", k);
             return false;
         }
         P.max_bounces = std::max(P.max_bounces, S.bounces);
-        const uint64_t tiles = uint64_t((S.width + 7u) / 8u) * ((S.height + 3u) / 4u);
-        const uint64_t work = P.work_base[k] + tiles * 32u, pix = P.pixel_base[k] + uint64_t(S.width) * S.height;
-        if (work > 0xffffffffull || pix > 0xffffffffull) { set_error(error, error_len, "batch too large"); return false; }
-        P.work_base[k + 1] = uint32_t(work);
-        P.pixel_base[k + 1] = uint32_t(pix);
+        total_work += scene_work(S);
+        const uint64_t pix = pixel_base[k] + uint64_t(S.width) * S.height;
+        if (total_work > 0xffffffffull || pix > 0xffffffffull) { set_error(error, error_len, "batch too large"); return false; }
+        pixel_base[k + 1] = uint32_t(pix);
         key = fnv(key, S.width);
         key = fnv(key, S.height);
         key = fnv(key, S.kind);
         key = fnv(key, S.iterations);
         key = fnv(key, S.bounces);
     }
+    P.scenes.reserve(count);
+    P.work_base.assign(count + 1, 0);
+    P.pixel_base.assign(count + 1, pixel_base[count]);
+    for (size_t k : work_order(scenes)) {
+        const size_t at = P.scenes.size();
+        P.work_base[at + 1] = P.work_base[at] + uint32_t(scene_work(scenes[k]));
+        P.pixel_base[at] = pixel_base[k];
+        P.scenes.push_back(scenes[k]);
+    }
     P.work = P.work_base[count];
-    P.pixels = P.pixel_base[count];
+    P.pixels = pixel_base[count];
     P.key = fnv(fnv(key, P.spp), count);
     return true;
 }
