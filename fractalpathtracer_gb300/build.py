@@ -42,7 +42,7 @@ def _units():
     units.append(("render_common.cu", "render_common.o", fast))
     # Voxel build and DDA: IEEE operations in source order (no contraction),
     # so brick tables and cell sequences are bit-identical to the CPU path.
-    units.append(("voxel.cu", "voxel.o", ["-fmad=false"]))
+    units.append(("voxel.cu", "voxel.o", ["-fmad=false", "-DFPT_IEEE_DIVISION"]))
     units.append(("mlp.cu", "mlp.o", []))
     units.append(("batch.cu", "batch.o", fast))
     units.append(("bridge.cu", "bridge.o", []))

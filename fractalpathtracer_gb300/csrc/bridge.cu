@@ -255,7 +255,14 @@ bool compile_scene(const FptRenderConfig &c, const FptCudaSceneExt *ext_in, Devi
     S.box_fixed2 = float(double(e.box_fixed_radius) * double(e.box_fixed_radius));
     S.box_min2 = float(double(e.box_min_radius) * double(e.box_min_radius));
     S.box_min_factor = S.box_min2 > 0.0f ? S.box_fixed2 / S.box_min2 : 1.0f;
-    S.box_fold_limit = e.box_fold_limit;
+    S.box_outer2 = std::max(S.box_min2, S.box_fixed2);
+    // A negative limit folds every coordinate, as 0 does (a coordinate of 0 is its own fold).
+    S.box_fold_limit = e.box_fold_limit < 0.0f ? 0.0f : e.box_fold_limit;
+    // Squared radius up to which an orbit is certainly inside the bailout radius: 2^-18 under its square, far above
+    // the square root's error (2^-22) and the rounding of the product.
+    const double bail = S.bailout > 0.0f ? S.bailout : std::max(S.set_values[2], 1.0f);
+    S.inside_r2 = float(std::min(bail * bail * (1.0 - 0x1p-18), 3.4e38));
+    if (!(S.inside_r2 >= 1.0e-30f)) S.inside_r2 = 0.0f;
     S.box_fold_value = e.box_fold_value;
     S.menger_scale = e.menger_scale;
     S.hybrid_period = e.hybrid_period;

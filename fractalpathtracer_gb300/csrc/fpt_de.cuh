@@ -9,10 +9,21 @@
 
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "fpt_math.cuh"
 #include "fpt_scene.h"
 
+// 1 / x as the unit's division rounds it (the voxel unit, FPT_IEEE_DIVISION,
+// divides exactly).
+#ifdef FPT_IEEE_DIVISION
+#define FPT_UNIT_RCP(x) __frcp_rn(x)
+#else
+#define FPT_UNIT_RCP(x) (1.0f / (x))
+#endif
+
 namespace fpt {
+
 
 struct Material {
     float3 rgb;
@@ -407,6 +418,31 @@ template <class T> __device__ __forceinline__ void box_step(T &x, T &y, T &z, T 
     x = x * s; y = y * s; z = z * s;
     dr = dr * T(fabsf(S.box_scale)) + T(1.0f);
 }
+// The same step in FP32 with fewer instructions and the same bits.  The fold's
+// signf(x) * val is val with the sign of x flipped in (x is not 0 where the
+// fold applies: the host clamps the limit to >= 0), and the two inner radii
+// share one branch (box_outer2 is the larger of their squares).  In the unit
+// with IEEE division a fixed radius of 1, the formula's default, takes the
+// correctly rounded reciprocal, which is the same number.
+__device__ __forceinline__ float box_fold(float x, float lim, uint32_t val) {
+    return fabsf(x) > lim ? __uint_as_float((__float_as_uint(x) & 0x80000000u) ^ val) - x : x;
+}
+__device__ __forceinline__ void box_step(float &x, float &y, float &z, float &dr, const DeviceScene &S) {
+    const float lim = S.box_fold_limit;
+    const uint32_t val = __float_as_uint(S.box_fold_value);
+    x = box_fold(x, lim, val);
+    y = box_fold(y, lim, val);
+    z = box_fold(z, lim, val);
+    const float r2 = x * x + y * y + z * z;
+    if (r2 < S.box_outer2) {
+        const float inv = S.box_fixed2 == 1.0f ? FPT_UNIT_RCP(r2) : S.box_fixed2 / r2;
+        const float f = r2 < S.box_min2 ? S.box_min_factor : inv;
+        x = x * f; y = y * f; z = z * f; dr = dr * f;
+    }
+    const float s = S.box_scale;
+    x = x * s; y = y * s; z = z * s;
+    dr = dr * fabsf(S.box_scale) + 1.0f;
+}
 // Menger fold step: abs, descending sort, scale about (1, 1, 1) with the
 // Menger-sponge z offset of orbit.rs:734-745.
 template <class T> __device__ __forceinline__ void menger_step(T &x, T &y, T &z, T &dr, float s) {
@@ -441,12 +477,8 @@ template <class T> __device__ __forceinline__ void orbit_start(Orbit<T> &o, T px
     o.escaped = false;
 }
 
-// One iteration; returns false once the orbit is finished (escaped, not
-// finite -- the step is rolled back -- or max_iter iterations done).
-template <int KIND, class T>
-__device__ __forceinline__ bool orbit_step(Orbit<T> &o, const DeviceScene &S, int max_iter, float bailout) {
-    const T ox = o.x, oy = o.y, oz = o.z;
-    const int i = o.i;
+// The formula's step and the added constant of iteration o.i (0-based).
+template <int KIND, class T> __device__ __forceinline__ void orbit_formula(Orbit<T> &o, const DeviceScene &S, int i) {
     bool add_c = true;
     if (KIND == KIND_BULB8) bulb8_step(o.x, o.y, o.z, o.dr, o.r);
     else if (KIND == KIND_BULB) {
@@ -461,6 +493,14 @@ __device__ __forceinline__ bool orbit_step(Orbit<T> &o, const DeviceScene &S, in
         else bulb_step(o.x, o.y, o.z, o.dr, o.r, S.power);
     }
     if (add_c) { o.x = o.x + o.cx; o.y = o.y + o.cy; o.z = o.z + o.cz; }
+}
+// One iteration; returns false once the orbit is finished (escaped, not
+// finite -- the step is rolled back -- or max_iter iterations done).
+template <int KIND, class T>
+__device__ __forceinline__ bool orbit_step(Orbit<T> &o, const DeviceScene &S, int max_iter, float bailout) {
+    const T ox = o.x, oy = o.y, oz = o.z;
+    const int i = o.i;
+    orbit_formula<KIND>(o, S, i);
     o.r = s_sqrt(o.x * o.x + o.y * o.y + o.z * o.z);
     o.i = i + 1;
     if (!isfinite(s_val(o.r))) {
@@ -490,14 +530,186 @@ template <int KIND, class T> __device__ __forceinline__ OrbitResult<T> orbit_fin
     return o;
 }
 
-template <int KIND, class T>
-__device__ __forceinline__ OrbitResult<T> orbit_eval(const DeviceScene &S, T px, T py, T pz, int max_iter, float bailout) {
-    Orbit<T> o;
-    orbit_start(o, px, py, pz);
-    if (max_iter > 0)
-        while (orbit_step<KIND>(o, S, max_iter, bailout)) {
+// The power-8 step of the hot kernels, operation by operation.  A path on a
+// fractal turns the last bit of a distance into another path, so each kernel
+// keeps the roundings that its compiled bulb8_step<float> had; they differ in
+// 1 / rho.  B8_TEMPLATE (every other kernel) is the template's loop.
+enum Bulb8Rounding : int {
+    B8_TEMPLATE = 0,
+    B8_RCP = 1,     // 1 / rho by reciprocal of the square root (primary rays, distance samples)
+    B8_RSQRT = 2,   // 1 / rho by reciprocal square root (the march kernel)
+};
+// For normal arguments the .ftz forms return the same bits as the others,
+// without the scaling that those have for denormals.
+__device__ __forceinline__ float sqrt_normal(float a) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float rcp_normal(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_normal(float a) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+constexpr float kSmallestNormal = 1.17549435e-38f;
+// Two floats in one register pair: the packed operations of this
+// architecture round each half as the scalar operation does.
+using float_pair = unsigned long long;
+__device__ __forceinline__ float_pair pair_of(float a, float b) {
+    float_pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void pair_parts(float_pair p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ float_pair pair_mul(float_pair a, float_pair b) {
+    float_pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float_pair pair_add(float_pair a, float_pair b) {
+    float_pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float_pair pair_fma(float_pair a, float_pair b, float_pair c) {
+    float_pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// The real parts (a) and doubled real parts (twice) of the squares of two
+// complex numbers with real parts a and imaginary parts b: each real part is
+// one fused operation on a rounded b^2.
+__device__ __forceinline__ void complex_square_real(float_pair &a, float_pair b, float_pair &twice) {
+    float p, q;
+    pair_parts(b, p, q);
+    const float_pair minus_b2 = pair_mul(b, pair_of(-p, -q));
+    twice = pair_add(a, a);
+    a = pair_fma(a, a, minus_b2);
+}
+// The step and the added constant; rho2 is at least kSmallestNormal.  The two
+// chains of squarings, (rho + i z)^8 and ((x + i y) / rho)^8, run side by side
+// in register pairs.
+__device__ __forceinline__ void bulb8_step_normal(Orbit<float> &o, float rho2, bool rsqrt) {
+    const float rho = sqrt_normal(rho2), inv = rsqrt ? rsqrt_normal(rho2) : rcp_normal(rho);
+    const float r2 = __fmul_rn(o.r, o.r);
+    const float r7 = __fmul_rn(__fmul_rn(__fmul_rn(r2, r2), r2), o.r);
+    o.dr = __fmaf_rn(__fmul_rn(r7, o.dr), 8.0f, 1.0f);
+    float_pair a = pair_of(rho, __fmul_rn(o.x, inv)), b = pair_of(o.z, __fmul_rn(o.y, inv)), a_twice;
+    complex_square_real(a, b, a_twice);
+    b = pair_mul(a_twice, b);
+    complex_square_real(a, b, a_twice);
+    b = pair_mul(a_twice, b);
+    complex_square_real(a, b, a_twice);
+    float a8, c8, a4_twice, u4_twice, b4, v4;
+    pair_parts(a, a8, c8);
+    pair_parts(a_twice, a4_twice, u4_twice);
+    pair_parts(b, b4, v4);
+    o.x = __fmaf_rn(a8, c8, o.cx);
+    o.y = __fmaf_rn(a8, __fmul_rn(u4_twice, v4), o.cy);
+    o.z = __fmaf_rn(a4_twice, b4, o.cz);
+}
+__device__ __forceinline__ float sum_squares(float x, float y, float z) { return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y))); }
+
+// One FP32 iteration: step, added constant, squared radius.  o.r is the radius
+// before it where the step uses the radius.
+template <int KIND>
+__device__ __forceinline__ float orbit_iterate(Orbit<float> &o, const DeviceScene &S, int b8) {
+    float r2;
+    if (KIND == KIND_BULB8) {
+        const float rho2 = __fmaf_rn(o.y, o.y, __fmul_rn(o.x, o.x));
+        if (rho2 >= kSmallestNormal) {
+            bulb8_step_normal(o, rho2, b8 == B8_RSQRT);
+        } else {
+            bulb8_step(o.x, o.y, o.z, o.dr, o.r);
+            o.x = o.x + o.cx; o.y = o.y + o.cy; o.z = o.z + o.cz;
         }
+        r2 = sum_squares(o.x, o.y, o.z);
+    } else {
+        orbit_formula<KIND>(o, S, o.i);
+        r2 = o.x * o.x + o.y * o.y + o.z * o.z;
+    }
+    ++o.i;
+    return r2;
+}
+// The orbit's position after n iterations from its start.
+template <int KIND> __device__ __noinline__ float3 orbit_position(const DeviceScene &S, float cx, float cy, float cz, int n, int b8) {
+    Orbit<float> o;
+    orbit_start(o, cx, cy, cz);
+    while (o.i < n) {
+        const float r2 = orbit_iterate<KIND>(o, S, b8);
+        if (KIND == KIND_BULB8) o.r = s_sqrt(r2);
+    }
+    return mk3(o.x, o.y, o.z);
+}
+
+// The FP32 orbit loop of the Mandelbox and the Menger fold, whose steps do not
+// use the radius, and of the power-8 Mandelbulb in the hot kernels.  One
+// comparison ends an iteration: of the squared radius with
+// DeviceScene::inside_r2, below which the orbit is inside whatever the square
+// root rounds to (Mandelbulb: of the radius with the bailout radius).  What
+// the loop stopped for is settled after it, where the warp's lanes are
+// together again: escaped, not finite (not-a-number fails the comparison too;
+// the step is rolled back by running the orbit to the iteration before), or
+// between inside_r2 and the bailout radius, where the loop goes on.
+// These kernels are bound by issued instructions (75-85% of cycles), and the
+// loop is most of them: 1024^3 Mandelbox staging 27.0 -> 16.3 ms, 333 x 217
+// Mandelbox frame 3.75 -> 2.89 ms, 1080p 16 spp Mandelbulb frame (device time)
+// 33.3 -> 28.5 ms, 720p Menger frame 18.1 -> 17.1 ms.  The formulas with
+// transcendental steps gain nothing from it (1.00-1.03x) and keep the
+// template's loop, as do kernels off the hot paths.
+template <int KIND>
+__device__ __forceinline__ OrbitResult<float> orbit_eval_f32(const DeviceScene &S, float px, float py, float pz, int max_iter, float bailout,
+                                                              int b8) {
+    Orbit<float> o;
+    orbit_start(o, px, py, pz);
+    float r2 = px * px + py * py + pz * pz;
+    if (KIND == KIND_BULB8) o.r = s_sqrt(sum_squares(px, py, pz));
+    while (true) {
+        bool inside = true;
+        while (inside && o.i < max_iter) {
+            r2 = orbit_iterate<KIND>(o, S, b8);
+            if (KIND == KIND_BULB8) {
+                o.r = s_sqrt(r2);
+                inside = o.r <= bailout;
+            } else {
+                inside = r2 <= S.inside_r2;
+            }
+        }
+        if (KIND != KIND_BULB8) o.r = s_sqrt(r2);
+        if (inside) break;
+        if (!isfinite(o.r)) {
+            const float3 p = orbit_position<KIND>(S, px, py, pz, o.i - 1, b8);
+            o.x = p.x; o.y = p.y; o.z = p.z;
+            if (KIND == KIND_BULB8) o.r = s_sqrt(__fadd_rn(__fmaf_rn(p.x, p.x, __fmul_rn(p.y, p.y)), __fmul_rn(p.z, p.z)));
+            else o.r = s_sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
+            break;
+        }
+        o.escaped = o.r > bailout;
+        if (o.escaped) break;
+    }
     return orbit_finish<KIND>(o);
+}
+
+template <int KIND, class T>
+__device__ __forceinline__ OrbitResult<T> orbit_eval(const DeviceScene &S, T px, T py, T pz, int max_iter, float bailout, int b8 = B8_TEMPLATE) {
+    if constexpr (std::is_same<T, float>::value && (KIND == KIND_BOX || KIND == KIND_MENGER)) {
+        return orbit_eval_f32<KIND>(S, px, py, pz, max_iter, bailout, b8);
+    } else {
+        if constexpr (std::is_same<T, float>::value && KIND == KIND_BULB8) {
+            if (b8 != B8_TEMPLATE) return orbit_eval_f32<KIND>(S, px, py, pz, max_iter, bailout, b8);
+        }
+        Orbit<T> o;
+        orbit_start(o, px, py, pz);
+        if (max_iter > 0)
+            while (orbit_step<KIND>(o, S, max_iter, bailout)) {
+            }
+        return orbit_finish<KIND>(o);
+    }
 }
 
 __device__ __forceinline__ int ext_iterations(const DeviceScene &S) {
@@ -510,17 +722,17 @@ __device__ __forceinline__ float ext_bailout(const DeviceScene &S) {
 // Extension formula as a Mandelbulber field (global transform, swizzle,
 // distance times world scale) or directly at p for the other scene ids.
 template <int KIND, class T>
-__device__ __forceinline__ OrbitResult<T> ext_field(const DeviceScene &S, T x, T y, T z, int mult) {
+__device__ __forceinline__ OrbitResult<T> ext_field(const DeviceScene &S, T x, T y, T z, int mult, int b8 = B8_TEMPLATE) {
     if (S.sdf_id == FPT_SDF_MANDELBULBER) {
         float ws = fmaxf(S.set_values[0], 1.0f);
         global_point(S, x, y, z);
         T inv = T(1.0f / ws);
-        OrbitResult<T> o = orbit_eval<KIND, T>(S, x / T(ws), z / T(ws), y / T(ws), ext_iterations(S) * max(mult, 1), ext_bailout(S));
+        OrbitResult<T> o = orbit_eval<KIND, T>(S, x / T(ws), z / T(ws), y / T(ws), ext_iterations(S) * max(mult, 1), ext_bailout(S), b8);
         (void)inv;
         o.d = o.d * T(ws);
         return o;
     }
-    return orbit_eval<KIND, T>(S, x, y, z, ext_iterations(S) * max(mult, 1), ext_bailout(S));
+    return orbit_eval<KIND, T>(S, x, y, z, ext_iterations(S) * max(mult, 1), ext_bailout(S), b8);
 }
 
 // deMandelbulber's iteration-threshold handling (shaders/Shaders.metal:970-994).
@@ -543,19 +755,19 @@ __device__ __forceinline__ Eval mandel_finish(const DeviceScene &S, float3 p, Fi
 }
 
 // Field sample (d, r, dr, +-iterations) of a Mandelbulber scene.
-template <int KIND> __device__ Field4 mandel_field(float3 p, const DeviceScene &S, int mult) {
+template <int KIND> __device__ Field4 mandel_field(float3 p, const DeviceScene &S, int mult, int b8 = B8_TEMPLATE) {
     if (KIND == KIND_GENERIC && S.formula == 0) return field_ifs(p, S, mult);
     OrbitResult<float> o;
     if (runtime_kind(KIND)) {
         switch (S.kind) {
-            case KIND_BULB8: o = ext_field<KIND_BULB8, float>(S, p.x, p.y, p.z, mult); break;
-            case KIND_BULB: o = ext_field<KIND_BULB, float>(S, p.x, p.y, p.z, mult); break;
-            case KIND_BOX: o = ext_field<KIND_BOX, float>(S, p.x, p.y, p.z, mult); break;
-            case KIND_MENGER: o = ext_field<KIND_MENGER, float>(S, p.x, p.y, p.z, mult); break;
-            default: o = ext_field<KIND_HYBRID, float>(S, p.x, p.y, p.z, mult); break;
+            case KIND_BULB8: o = ext_field<KIND_BULB8, float>(S, p.x, p.y, p.z, mult, b8); break;
+            case KIND_BULB: o = ext_field<KIND_BULB, float>(S, p.x, p.y, p.z, mult, b8); break;
+            case KIND_BOX: o = ext_field<KIND_BOX, float>(S, p.x, p.y, p.z, mult, b8); break;
+            case KIND_MENGER: o = ext_field<KIND_MENGER, float>(S, p.x, p.y, p.z, mult, b8); break;
+            default: o = ext_field<KIND_HYBRID, float>(S, p.x, p.y, p.z, mult, b8); break;
         }
     } else {
-        o = ext_field<KIND, float>(S, p.x, p.y, p.z, mult);
+        o = ext_field<KIND, float>(S, p.x, p.y, p.z, mult, b8);
     }
     return {o.d, o.r, o.dr, o.escaped ? -float(o.iterations) : float(o.iterations)};
 }
@@ -856,18 +1068,18 @@ enum EvalMode : int {
 };
 
 template <int KIND>
-__device__ __forceinline__ Eval ext_eval(const DeviceScene &S, float3 p) {
+__device__ __forceinline__ Eval ext_eval(const DeviceScene &S, float3 p, int b8 = B8_TEMPLATE) {
     Eval e;
     if (S.sdf_id == FPT_SDF_MANDELBULBER) {
-        e = mandel_finish(S, p, mandel_field<KIND>(p, S, 1));
+        e = mandel_finish(S, p, mandel_field<KIND>(p, S, 1, b8));
     } else {
         OrbitResult<float> o;
         switch (runtime_kind(KIND) ? S.kind : (uint32_t)KIND) {
-            case KIND_BULB8: o = orbit_eval<KIND_BULB8, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S)); break;
-            case KIND_BULB: o = orbit_eval<KIND_BULB, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S)); break;
-            case KIND_BOX: o = orbit_eval<KIND_BOX, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S)); break;
-            case KIND_MENGER: o = orbit_eval<KIND_MENGER, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S)); break;
-            default: o = orbit_eval<KIND_HYBRID, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S)); break;
+            case KIND_BULB8: o = orbit_eval<KIND_BULB8, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S), b8); break;
+            case KIND_BULB: o = orbit_eval<KIND_BULB, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S), b8); break;
+            case KIND_BOX: o = orbit_eval<KIND_BOX, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S), b8); break;
+            case KIND_MENGER: o = orbit_eval<KIND_MENGER, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S), b8); break;
+            default: o = orbit_eval<KIND_HYBRID, float>(S, p.x, p.y, p.z, ext_iterations(S), ext_bailout(S), b8); break;
         }
         e = {o.d, float(o.iterations) / float(max(ext_iterations(S), 1)), 0, o.iterations};
     }
@@ -881,7 +1093,7 @@ __device__ __forceinline__ Eval ext_eval(const DeviceScene &S, float3 p) {
 // One evaluation of the scene at p.  KIND selects a specialised estimator;
 // KIND_GENERIC dispatches on the scene at run time.
 template <int KIND>
-__device__ __forceinline__ Eval scene_eval(const DeviceScene &S, float3 p, int mode) {
+__device__ __forceinline__ Eval scene_eval(const DeviceScene &S, float3 p, int mode, int b8 = B8_TEMPLATE) {
     Eval e;
     if (KIND != KIND_GENERIC || S.formula != 0) {
         if (mode == EV_NORMAL && S.sdf_id == FPT_SDF_MANDELBULBER) {
@@ -889,7 +1101,7 @@ __device__ __forceinline__ Eval scene_eval(const DeviceScene &S, float3 p, int m
             Field4 f = mandel_field<KIND>(p, S, mult);
             return {f.d, 0.0f, 0};
         }
-        e = ext_eval<KIND>(S, p);
+        e = ext_eval<KIND>(S, p, b8);
     } else {
         switch (S.sdf_id) {
             case FPT_SDF_PROGRAM:

@@ -236,13 +236,13 @@ __device__ __noinline__ float3 normal_fp64(const DeviceScene &S, double px, doub
 }
 
 // Plain-loop march (focus prepass, primary rays, diagnostics).
-template <int KIND>
+template <int KIND, int B8 = B8_TEMPLATE>
 __device__ March march_loop(const DeviceScene &S, float3 origin, float3 dir, int ni, float min_dist, float lod_falloff) {
     March m;
     TranslucencyProbe<KIND> probe{&S};
     bool more = march_begin(m, S, origin, dir, ni, min_dist, lod_falloff);
     while (more) {
-        float d = scene_eval<KIND>(S, m.pos, EV_MAP).d;
+        float d = scene_eval<KIND>(S, m.pos, EV_MAP, B8).d;
         more = march_update(m, S, d, probe);
     }
     return m;

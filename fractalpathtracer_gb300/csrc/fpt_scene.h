@@ -84,6 +84,8 @@ struct DeviceScene {
     float bailout;
     float power;
     float box_scale, box_fixed2, box_min2, box_min_factor, box_fold_limit, box_fold_value;
+    float box_outer2;          // max(box_min2, box_fixed2)
+    float inside_r2;           // an orbit whose squared radius is at most this has not escaped, whatever the square root rounds to
     float menger_scale;
     uint32_t hybrid_period;
     uint32_t ground_plane;

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(128) trace_primary_kernel(const DeviceScene *s
     FptCudaPrimaryHit h;
     h.distance = 0.0f; h.normal[0] = h.normal[1] = h.normal[2] = 0.0f; h.steps = 0; h.hit = 0;
     if (camera_ray(S, uv, rng, false, rp, dr)) {
-        March m = march_loop<KIND>(S, rp, dr, int(S.render[1]), S.render[3], 0.0002f);
+        March m = march_loop<KIND, B8_RCP>(S, rp, dr, int(S.render[1]), S.render[3], 0.0002f);
         float travel = len3(m.pos - rp);
         bool hit = m.found && isfinite(travel) && travel < S.render[4] * 0.99f;
         int steps = m.steps;
@@ -208,7 +208,7 @@ __global__ void sample_distance_kernel(const DeviceScene *scene, const float4 *p
     const DeviceScene &S = *scene;
     float4 p4 = points[i];
     float3 p = mk3(p4.x, p4.y, p4.z);
-    Eval e = scene_eval<KIND>(S, p, EV_RAW);
+    Eval e = scene_eval<KIND>(S, p, EV_RAW, B8_RCP);
     float dr = 0.0f, it = 0.0f;
     if (S.sdf_id == FPT_SDF_MANDELBULBER) {
         Field4 f = mandel_field<KIND>(p, S, 1);

@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
         TranslucencyProbe<KIND> probe{sp};
         // One distance evaluation for every lane with a march in flight.
         if (active) {
-            const Eval ev = have_d ? Eval{known_d, 0.0f, 0, 0} : scene_eval<KIND>(S, m.pos, EV_MAP);
+            const Eval ev = have_d ? Eval{known_d, 0.0f, 0, 0} : scene_eval<KIND>(S, m.pos, EV_MAP, KIND == KIND_BULB8 ? B8_RSQRT : B8_TEMPLATE);
             const float d = ev.d;
             c_job_orbit += uint32_t(ev.iters);
             have_d = false;

@@ -107,3 +107,47 @@ def test_mandelbulb_power2_triplex_field(native):
     ok = (nr > 1e-6) & np.isfinite(ng) & (np.abs(r[:, 0]) > 1e-3)
     cosang = (gg[ok] * gr[ok]).sum(1) / (ng[ok] * nr[ok])
     assert np.percentile(np.degrees(np.arccos(np.clip(cosang, -1, 1))), 99) < 0.5
+
+
+def _bulb8_f32(points, iterations, bailout):
+    """The algebraic power-8 orbit in FP32: (rho + i z)^8 times ((x + i y) / rho)^8, as the kernels compute it."""
+    f = np.float32
+    out = np.zeros(len(points))
+    for k, (px, py, pz) in enumerate(points[:, [0, 2, 1]].astype(f)):   # the field's axes: world x, z, y
+        x, y, z, dr = px, py, pz, f(1)
+        r = np.sqrt(x * x + y * y + z * z)
+        for _ in range(iterations):
+            rho = np.sqrt(x * x + y * y)
+            w, e = np.array([rho, z], f), np.array([x / rho, y / rho] if rho > 0 else [1, 0], f)
+            for _ in range(3):
+                w = np.array([w[0] * w[0] - w[1] * w[1], 2 * w[0] * w[1]], f)
+                e = np.array([e[0] * e[0] - e[1] * e[1], 2 * e[0] * e[1]], f)
+            dr = r ** f(7) * dr * f(8) + f(1)
+            x, y, z = w[0] * e[0] + px, w[0] * e[1] + py, w[1] + pz
+            r = np.sqrt(x * x + y * y + z * z)
+            if r > bailout:
+                break
+        out[k] = 0.5 * r * np.log(r) / dr if r > 1 else 0.0
+    return out
+
+
+@pytest.mark.parametrize("iterations,bailout", [(1, 2.0), (2, 1.0), (8, 2.0), (5, 50.0)])
+def test_mandelbulb8_step_edges(native, iterations, bailout):
+    """The power-8 step's branches: the polar axis (x = y = 0), coordinate planes, the origin, points whose squares
+    are denormal or zero, and orbits that stop at the first iteration or never escape."""
+    cfg, ext = scenes.mandelbulb_primary(8, 8)
+    ext.iterations, ext.bailout = iterations, bailout
+    p = pts(4096, -1.4, 1.4, seed=3)
+    p[:512, 0] = 0.0
+    p[256:768, 2] = 0.0          # the field's y: with the first lines, points of the polar axis
+    p[768:1024, 1] = 0.0
+    p[1024:1536, :3] *= np.float32(1e-19)
+    p[1536:1792, 0] *= np.float32(1e-22)
+    p[1536:1792, 2] *= np.float32(1e-22)
+    p[1792, :3] = 0.0
+    g = native.sample_distance(cfg, ext, p)
+    r = oracle.sample_distance(cfg, ext, p, fp64=True)
+    flat = slice(1536, 1792)     # x^2 + y^2 is denormal: FP32 has no angle left there, so FP32 is the reference
+    r[flat, 0] = _bulb8_f32(p[flat], iterations, bailout)
+    _gate(g[:, 0], r[:, 0], outliers=5e-3)
+    assert np.mean(g[:, 3] == r[:, 3]) > 0.995

@@ -120,3 +120,28 @@ def test_voxel_path_render_through_drop_in(native, tmp_path):
     dense.voxel_storage = ffi.VOXEL_STORAGE_DENSE
     res_dense = native.metal_render(dense, str(tmp_path / "d.png"))
     assert np.array_equal(res["linear"], res_dense["linear"])
+
+
+@pytest.mark.parametrize("change", [
+    {},                                                          # fixed radius 1: the reciprocal
+    {"box_fixed_radius": 1.3},                                   # the general division
+    {"box_fixed_radius": 0.4, "box_min_radius": 0.5},            # minimum radius above the fixed one
+    {"box_fold_limit": 0.0, "box_fold_value": 1.5}, {"box_fold_limit": -0.5, "box_fold_value": -1.0},
+    {"iterations": 1}, {"bailout": 2.0}, {"bailout": 1e-3},      # orbits that stop early
+    {"iterations": 200, "bailout": 1e30, "box_scale": 2.2},      # a squared radius that overflows: the step is rolled back
+    {"formula": ffi.FORMULA_MENGER_FOLD, "menger_scale": 3.0, "iterations": 5, "bailout": 1e6},
+    {"formula": ffi.FORMULA_MENGER_FOLD, "menger_scale": 2.5, "iterations": 9, "bailout": 3.0},
+], ids=lambda c: "-".join(f"{k}={v}" for k, v in c.items()) or "plain")
+def test_orbit_loop_bit_exact(native, change):
+    """Brick tables and fp16 distances of the Mandelbox's and the Menger fold's FP32 loop, bit for bit, over the forms
+    of its step and the ways an orbit ends."""
+    cfg, ext = scenes.voxel_mandelbox(40, 8, 8)
+    for name, value in change.items():
+        setattr(ext, name, value)
+    info = native_ext.voxel_build(cfg, ext, 8)
+    t, o, d, _ = native_ext.voxel_read(info)
+    rt, ro, rd, _, rcells = oracle.voxel_build(cfg, ext, 8)
+    assert info["active_cells"] == rcells
+    assert np.array_equal(t, rt)
+    if rcells:
+        assert np.array_equal(o, ro) and np.array_equal(d, rd)
