@@ -108,15 +108,19 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
     __syncthreads();
     return warp_prefix + x - v;
 }
+// `reach` (optional, zeroed): the box of the occupied bricks, as the largest
+// ~coordinate (words 0-2) and the largest coordinate plus one (words 3-5).
 __global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(const uint32_t *count, uint32_t n, uint32_t *offset,
-                                                                   uint32_t *block_sums) {
+                                                                   uint32_t *block_sums, uint32_t brick_grid, uint32_t *reach) {
     __shared__ uint32_t smem[32];
+    __shared__ uint32_t s_reach[6];
     uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
     uint32_t f[kScanPer], s = 0;
     for (int k = 0; k < kScanPer; ++k) {
         f[k] = (base + k < n && count[base + k] > 0u) ? 1u : 0u;
         s += f[k];
     }
+    if (reach && threadIdx.x < 6u) s_reach[threadIdx.x] = 0u;
     uint32_t total;
     uint32_t pre = block_exclusive_scan(s, smem, total);
     for (int k = 0; k < kScanPer; ++k) {
@@ -124,6 +128,19 @@ __global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(const uint32_
         pre += f[k];
     }
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
+    if (reach && total > 0u) {   // the same in every thread
+        for (int k = 0; k < kScanPer; ++k) {
+            if (f[k] == 0u) continue;
+            const uint32_t b = base + k;
+            const uint32_t c[3] = {b % brick_grid, (b / brick_grid) % brick_grid, b / (brick_grid * brick_grid)};
+            for (int a = 0; a < 3; ++a) {
+                atomicMax(&s_reach[a], ~c[a]);
+                atomicMax(&s_reach[3 + a], c[a] + 1u);
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 6u) atomicMax(&reach[threadIdx.x], s_reach[threadIdx.x]);
+    }
 }
 __global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(uint32_t *block_sums, uint32_t nblocks, uint32_t *grand_total) {
     __shared__ uint32_t smem[32];
@@ -535,6 +552,7 @@ struct VoxelState {
     bool built = false;
     uint32_t format = 0, brick_size = 0, res = 0, brick_grid = 0, active_bricks = 0;
     uint64_t active_cells = 0, memory_bytes = 0;
+    int occ_lo[3] = {1, 1, 1}, occ_hi[3] = {0, 0, 0};   // box of cells that holds every occupied brick (occupancy bricks)
     float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0}, cs[3] = {0, 0, 0};
     uint32_t *table = nullptr; size_t cap_table = 0;
     uint32_t *count = nullptr; size_t cap_count = 0;
@@ -568,6 +586,7 @@ static vox::Grid grid_view() {
     g.occ = V.occ;
     g.mask = reinterpret_cast<const uint64_t *>(V.mask);
     g.cells = V.cells;
+    for (int k = 0; k < 3; ++k) { g.occ_lo[k] = V.occ_lo[k]; g.occ_hi[k] = V.occ_hi[k]; }
     return g;
 }
 
@@ -585,18 +604,25 @@ static bool launch_build(const DeviceScene *scene, const VoxBuild &B, uint32_t b
         brick_classify_kernel<KIND, 4><<<nb, 64, 0, st>>>(scene, B, V.count, V.stats);
     }
     uint32_t nblocks = (nb + kScanBlock - 1) / kScanBlock;
-    scan_blocks_kernel<<<nblocks, kScanThreads, 0, st>>>(V.count, nb, V.offset, V.sums);
+    uint32_t *const reach = format == VF_OCCUPANCY ? reinterpret_cast<uint32_t *>(V.stats + 2) : nullptr;
+    scan_blocks_kernel<<<nblocks, kScanThreads, 0, st>>>(V.count, nb, V.offset, V.sums, B.brick_grid, reach);
     scan_sums_kernel<<<1, kScanThreads, 0, st>>>(V.sums, nblocks, reinterpret_cast<uint32_t *>(V.stats + 1));
     scan_add_kernel<<<(nb + 255) / 256, 256, 0, st>>>(V.offset, nb, V.sums);
     if (!check(cudaGetLastError(), "voxel classify/scan launch", error, error_len)) return false;
     // Size the payload from the active-brick total.
-    unsigned long long host_stats[2] = {0, 0};
+    unsigned long long host_stats[5] = {0, 0, 0, 0, 0};   // active cells; active bricks; their box
     if (!check(cudaMemcpyAsync(host_stats, V.stats, sizeof(host_stats), cudaMemcpyDeviceToHost, st), "voxel count readback", error,
                error_len))
         return false;
     if (!check(cudaStreamSynchronize(st), "voxel classification", error, error_len)) return false;
     V.active_cells = host_stats[0];
     V.active_bricks = uint32_t(host_stats[1] & 0xffffffffull);
+    uint32_t box[6];
+    std::memcpy(box, host_stats + 2, sizeof(box));
+    for (int k = 0; k < 3; ++k) {
+        V.occ_lo[k] = V.active_bricks ? int(~box[k] * bs) : 1;
+        V.occ_hi[k] = V.active_bricks ? int(std::min(box[3 + k] * bs, B.res)) - 1 : 0;
+    }
     const size_t cells = std::max<size_t>(1, size_t(V.active_bricks) * bs * bs * bs);
     if (format == VF_OCCUPANCY) {
         if (!ensure_buffer((void **)&V.occ, &V.cap_occ, cells, error, error_len)) return false;
@@ -1085,7 +1111,7 @@ extern "C" int fpt_cuda_voxel_build_static(const struct FptRenderConfig *config,
     if (S.kind == KIND_BOX) brick_classify_kernel<KIND_BOX, 8><<<nb, 512, 0, st>>>(&sc->scene, B, sc->count, sc->stats);
     else brick_classify_kernel<KIND_GENERIC, 8><<<nb, 512, 0, st>>>(&sc->scene, B, sc->count, sc->stats);
     const uint32_t nblocks = (nb + kScanBlock - 1) / kScanBlock;
-    scan_blocks_kernel<<<nblocks, kScanThreads, 0, st>>>(sc->count, nb, sc->offset, sc->sums);
+    scan_blocks_kernel<<<nblocks, kScanThreads, 0, st>>>(sc->count, nb, sc->offset, sc->sums, bg, nullptr);
     scan_sums_kernel<<<1, kScanThreads, 0, st>>>(sc->sums, nblocks, reinterpret_cast<uint32_t *>(sc->stats + 1));
     scan_add_kernel<<<(nb + 255) / 256, 256, 0, st>>>(sc->offset, nb, sc->sums);
     if (!check(cudaGetLastError(), "classification launch", error, error_len)) return 1;

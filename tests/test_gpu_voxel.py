@@ -145,3 +145,31 @@ def test_orbit_loop_bit_exact(native, change):
     assert np.array_equal(t, rt)
     if rcells:
         assert np.array_equal(o, ro) and np.array_equal(d, rd)
+
+
+@pytest.mark.parametrize("eye,bounds", [
+    ((5.5, 4.0, -9.0), (-4.0, 4.0)), ((0.0, 0.0, -9.0), (-4.0, 4.0)),   # outside, and along an axis
+    ((0.1, 0.2, 0.3), (-4.0, 4.0)), ((3.5, 3.5, -3.5), (-4.0, 4.0)),    # inside the occupied box, in an empty corner
+    ((-6.0, 0.5, 0.0), (-2.02, 2.02)), ((3.0, 3.0, 3.0), (-1.0, 3.0)),  # bricks up to the grid's faces
+    ((40.0, -900.0, 30.0), (-4.0, 4.0)),                                # crossing times far above a cell's
+    ((5.5, 4.0, -9.0), (3.0, 4.0)),                                     # a grid with no occupied brick
+])
+@pytest.mark.parametrize("resolution", [60, 203])
+def test_occupied_box_traversal_bit_exact(native, eye, bounds, resolution):
+    """Primary and shadow hits where the traversal starts, ends or passes outside the box of the occupied bricks."""
+    cfg, ext = scenes.voxel_mandelbox(resolution, 97, 61)
+    cfg.voxel_bounds_min[:] = [bounds[0]] * 3
+    cfg.voxel_bounds_max[:] = [bounds[1]] * 3
+    scenes.look_at(cfg, eye, (0.0, 0.0, 0.0))
+    if max(abs(v) for v in eye) > 100.0:
+        cfg.camera_fov = 2.0
+    native_ext.voxel_build(cfg, ext, 8)
+    h, _, _ = native_ext.voxel_render(cfg, ext, image=False)
+    rt, ro, _, _, _ = oracle.voxel_build(cfg, ext, 8)
+    ref = oracle.voxel_primary(cfg, ext, rt, ro)
+    hit = h["t"] >= 0
+    assert np.array_equal(h["t"], ref[..., 0].astype(np.float32))
+    assert np.array_equal(h["cell"][hit].astype(np.float64), ref[..., 1][hit])
+    assert np.array_equal(h["lit"].astype(np.float64), ref[..., 2])
+    assert np.array_equal(h["steps"].astype(np.float64), ref[..., 3])
+    assert np.array_equal(h["shadow_steps"].astype(np.float64), ref[..., 4])
