@@ -269,8 +269,9 @@ bool capture_pass(const BatchPlan &P, const MarchVariant &V, uint32_t wave_paths
     return check(e, "graph instantiation", error, error_len);
 }
 
-// Renders all spp passes with one graph; returns the device time of the replays.
-bool render_plan(const BatchPlan &P, const TuneChoice &choice, float &ms, uint32_t &launches_per_pass, double &build_ms,
+// Renders all spp passes with one graph; returns the device time of the replays.  `linear` / `rgba`: the caller's
+// result arrays (populated meanwhile), or null.
+bool render_plan(const BatchPlan &P, const TuneChoice &choice, float *linear, uint8_t *rgba, float &ms, uint32_t &launches_per_pass, double &build_ms,
                  char *error, size_t error_len) {
     Context &c = ctx();
     BatchState &B = bstate();
@@ -302,6 +303,7 @@ bool render_plan(const BatchPlan &P, const TuneChoice &choice, float &ms, uint32
         cudaEventRecord(e0, c.stream);
         for (uint32_t s = 0; s < P.spp && good; ++s) good = check(cudaGraphLaunch(exec, c.stream), "graph launch", error, error_len);
         cudaEventRecord(e1, c.stream);
+        if (good) populate_pages({{linear, P.pixels * sizeof(float4)}, {rgba, P.pixels * 4}});
         good = good && check(cudaStreamSynchronize(c.stream), "batch render", error, error_len);
         if (good) cudaEventElapsedTime(&ms, e0, e1);
         uint32_t guard = 0;
@@ -341,7 +343,7 @@ int fpt_cuda_render_batch(const struct FptRenderConfig *configs, const struct Fp
     float ms = 0.0f;
     uint32_t launches = 0;
     double build_ms = 0.0;
-    if (!render_plan(P, choice, ms, launches, build_ms, error, error_len)) return 1;
+    if (!render_plan(P, choice, linear_output, rgba_output, ms, launches, build_ms, error, error_len)) return 1;
     Context &c = ctx();
     BatchState &B = bstate();
     if (linear_output &&
@@ -398,7 +400,7 @@ int fpt_cuda_autotune_batch(const struct FptRenderConfig *configs, const struct 
             float ms = 0.0f;
             uint32_t launches = 0;
             double build_ms = 0.0;
-            if (!render_plan(P, cd.choice, ms, launches, build_ms, error, error_len)) return 1;
+            if (!render_plan(P, cd.choice, nullptr, nullptr, ms, launches, build_ms, error, error_len)) return 1;
             if (r >= 0) cd.ms.push_back(ms);
         }
     auto median = [](std::vector<float> v) {

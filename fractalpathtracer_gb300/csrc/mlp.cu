@@ -1069,6 +1069,7 @@ int fpt_cuda_mlp_predict(uint64_t model, const float *points_xyzw, size_t n, flo
         const unsigned blocks = unsigned(std::min<size_t>((n + 127) / 128, size_t(sms) * 8));
         mlp::predict_kernel<<<blocks, 128, mlp::forward_smem_bytes(), c.stream>>>(hm->view(), c.points, c.grads, uint32_t(n));
     }
+    populate_pages({{distances, n * sizeof(float)}});
     if (!check(cudaGetLastError(), "prediction launch", error, error_len) ||
         !check(cudaMemcpyAsync(distances, c.grads, n * sizeof(float), cudaMemcpyDeviceToHost, c.stream), "prediction readback", error, error_len))
         return 1;

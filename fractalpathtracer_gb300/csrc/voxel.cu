@@ -777,6 +777,7 @@ int voxel_render_core(const FptRenderConfig &config, const FptCudaSceneExt *ext,
                                                        config.voxel_offset_mode);
     if (!check(launch_present(c.scene, S.width, S.height, c.accum, c.rgba, c.stream), "present launch", error, error_len)) return 1;
     cudaEventRecord(c.ev1, c.stream);
+    populate_pages({{linear_output, pixels * sizeof(float4)}, {rgba_output, pixels * 4}});
     if (!check(cudaStreamSynchronize(c.stream), "voxel render", error, error_len)) return 1;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c.ev0, c.ev1);
@@ -867,6 +868,7 @@ int fpt_cuda_dda_sequence(const float *rays, size_t ray_count, uint32_t capacity
     if (!check(cudaMemcpyAsync(V.rays, rays, size_t(n) * 24, cudaMemcpyHostToDevice, c.stream), "ray upload", error, error_len)) return 1;
     dda_sequence_kernel<<<(n + 127) / 128, 128, 0, c.stream>>>(grid_view(), V.rays, n, want_seq ? capacity : 0,
                                                               want_seq ? V.seq : nullptr, V.seq_len, V.hits);
+    populate_pages({{hits, size_t(n) * sizeof(FptCudaVoxelHit)}, {want_seq ? sequence : nullptr, size_t(n) * capacity * 4}});
     if (!check(cudaStreamSynchronize(c.stream), "DDA sequence", error, error_len)) return 1;
     if (!check(cudaMemcpy(hits, V.hits, size_t(n) * sizeof(FptCudaVoxelHit), cudaMemcpyDeviceToHost), "hit readback", error, error_len))
         return 1;
@@ -969,6 +971,7 @@ int fpt_cuda_voxel_render(const struct FptRenderConfig *config, const struct Fpt
     voxel_primary_kernel<<<grid, 128, 0, c.stream>>>(grid_view(), exact_camera(*config), config->width, config->height,
                                                     make_float3(sun[0], sun[1], sun[2]), eps, V.hits, c.rgba);
     cudaEventRecord(c.ev1, c.stream);
+    populate_pages({{hits, pixels * sizeof(FptCudaVoxelHit)}, {rgba, pixels * 4}});
     if (!check(cudaStreamSynchronize(c.stream), "voxel primary render", error, error_len)) return 1;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c.ev0, c.ev1);

@@ -116,7 +116,7 @@ def metal_render(config: ffi.FptRenderConfig, output_path: str, linear_output: b
     vmem, vbricks, vcells, vrej, scs = C.c_uint64(), C.c_uint32(), C.c_uint64(), C.c_uint32(), C.c_uint32()
     bgs, svs, sps, prof = ffi.FptBoundGridStats(), ffi.FptStitchValidationStats(), ffi.FptStitchPipelineStats(), ffi.FptSdfProfileStats()
     n = config.width * config.height * 4
-    lin = np.zeros(n, np.float32) if linear_output else None
+    lin = np.empty(n, np.float32) if linear_output else None
     e = _err()
     rc = L.fpt_metal_render(b"", b"", b"", _b(output_path), None, 0, C.byref(config), C.byref(build_ms), C.byref(elapsed),
                             C.byref(vmem), C.byref(vbricks), C.byref(vcells), C.byref(vrej), C.byref(bgs), C.byref(scs),
@@ -144,8 +144,8 @@ def cuda_render(config: ffi.FptRenderConfig, ext: ffi.FptCudaSceneExt | None = N
     for a, dt in ((out_linear, np.float32), (out_rgba, np.uint8)):
         if a is not None and (a.dtype != dt or a.size != n or not a.flags["C_CONTIGUOUS"]):
             raise ValueError(f"output array must be a contiguous {np.dtype(dt).name} array of {n} elements")
-    lin = (out_linear.reshape(-1) if out_linear is not None else np.zeros(n, np.float32)) if linear else None
-    rgba = out_rgba.reshape(-1) if out_rgba is not None else np.zeros(n, np.uint8)
+    lin = (out_linear.reshape(-1) if out_linear is not None else np.empty(n, np.float32)) if linear else None
+    rgba = out_rgba.reshape(-1) if out_rgba is not None else np.empty(n, np.uint8)
     elapsed = C.c_double()
     prof = ffi.FptSdfProfileStats()
     e = _err()
@@ -167,7 +167,7 @@ def trace_primary(config: ffi.FptRenderConfig, ext: ffi.FptCudaSceneExt | None =
     """fpt_cuda_trace_primary: (H, W) structured array (row 0 = bottom) and elapsed ms."""
     L = lib()
     n = config.width * config.height
-    hits = np.zeros(n, HIT_DTYPE)
+    hits = np.empty(n, HIT_DTYPE)
     elapsed = C.c_double()
     e = _err()
     rc = L.fpt_cuda_trace_primary(C.byref(config), C.byref(ext) if ext is not None else None,
@@ -181,7 +181,7 @@ def sample_field(config: ffi.FptRenderConfig, points: np.ndarray) -> np.ndarray:
     """fpt_mandelbulber_sample_field: (n, 4) {distance, radius, derivative, iterations}."""
     L = lib()
     pts = np.ascontiguousarray(points, np.float32).reshape(-1, 4)
-    out = np.zeros((len(pts), 4), np.float32)
+    out = np.empty((len(pts), 4), np.float32)
     e = _err()
     rc = L.fpt_mandelbulber_sample_field(b"", None, 0, C.byref(config), _ptr(pts, C.c_float), len(pts),
                                          out.ctypes.data_as(C.POINTER(ffi.FptMandelbulberFieldSample)), e, len(e))
@@ -194,8 +194,8 @@ def sample_distance(config: ffi.FptRenderConfig, ext: ffi.FptCudaSceneExt | None
     """fpt_cuda_sample_distance: (n, 4) {distance, orbit, derivative, iterations} [and (n, 3) gradients]."""
     L = lib()
     pts = np.ascontiguousarray(points, np.float32).reshape(-1, 4)
-    out = np.zeros((len(pts), 4), np.float32)
-    g = np.zeros((len(pts), 3), np.float32) if gradients else None
+    out = np.empty((len(pts), 4), np.float32)
+    g = np.empty((len(pts), 3), np.float32) if gradients else None
     e = _err()
     rc = L.fpt_cuda_sample_distance(C.byref(config), C.byref(ext) if ext is not None else None, _ptr(pts, C.c_float),
                                     len(pts), _ptr(out, C.c_float), _ptr(g, C.c_float) if g is not None else None, e, len(e))

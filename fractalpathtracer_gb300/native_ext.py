@@ -142,7 +142,7 @@ def dda_sequence(rays: np.ndarray, capacity: int = 0):
     from .native import lib
     r = np.ascontiguousarray(rays, np.float32).reshape(-1, 6)
     n = len(r)
-    hits = np.zeros(n, VOXEL_HIT_DTYPE)
+    hits = np.empty(n, VOXEL_HIT_DTYPE)
     seq = np.zeros((n, capacity), np.uint32) if capacity else None
     seq_len = np.zeros(n, np.uint32) if capacity else None
     e = _err()
@@ -156,8 +156,8 @@ def dda_sequence(rays: np.ndarray, capacity: int = 0):
 def voxel_render(cfg, ext=None, image=True):
     from .native import lib
     n = cfg.width * cfg.height
-    hits = np.zeros(n, VOXEL_HIT_DTYPE)
-    rgba = np.zeros((cfg.height, cfg.width, 4), np.uint8) if image else None
+    hits = np.empty(n, VOXEL_HIT_DTYPE)
+    rgba = np.empty((cfg.height, cfg.width, 4), np.uint8) if image else None
     ms = C.c_double()
     e = _err()
     _check(lib().fpt_cuda_voxel_render(C.byref(cfg), C.byref(ext) if ext is not None else None,
@@ -215,7 +215,7 @@ def _f32(a):
 def mlp_predict(handle: int, points) -> np.ndarray:
     from .native import lib
     pts = np.ascontiguousarray(points, np.float32).reshape(-1, 4)
-    out = np.zeros(len(pts), np.float32)
+    out = np.empty(len(pts), np.float32)
     e = _err()
     _check(lib().fpt_cuda_mlp_predict(handle, _f32(pts), len(pts), _f32(out), e, len(e)), e)
     return out
@@ -280,8 +280,8 @@ def render_batch(bundles, linear=True, rgba=False):
     cfgs, exts = _batch_arrays(bundles)
     sizes = [(b.cfg.height, b.cfg.width) for b in bundles]
     total = sum(h * w for h, w in sizes)
-    lin = np.zeros(total * 4, np.float32) if linear else None
-    img = np.zeros(total * 4, np.uint8) if rgba else None
+    lin = np.empty(total * 4, np.float32) if linear else None
+    img = np.empty(total * 4, np.uint8) if rgba else None
     st = FptCudaBatchStats()
     e = _err()
     _check(lib().fpt_cuda_render_batch(cfgs, exts, len(bundles),

@@ -197,3 +197,18 @@ def test_loop_time_limit(native):
         nx.set_loop_limit(0)
     _, after, _ = native.cuda_render(b.cfg, b.ext, linear=False)
     assert np.array_equal(before, after)
+
+
+@pytest.mark.parametrize("width,height,offset", [(16, 8, 0), (640, 360, 12345), (1031, 517, 1)])
+def test_results_into_part_of_an_array(native, width, height, offset):
+    """Results land in caller-owned arrays that start and end anywhere in a page, fresh or not; the bytes around them stay."""
+    b = scenes.mandelbulb_path(width, height, 1)
+    want, want_img, _ = native.cuda_render(b.cfg, b.ext)
+    n = width * height * 4
+    lin, img = np.zeros(n + offset + 7, np.float32), np.empty(n + offset + 7, np.uint8)
+    img[:offset] = 7
+    img[offset + n:] = 9
+    got, got_img, _ = native.cuda_render(b.cfg, b.ext, out_linear=lin[offset:offset + n], out_rgba=img[offset:offset + n])
+    assert np.array_equal(got, want) and np.array_equal(got_img, want_img)
+    assert not lin[:offset].any() and not lin[offset + n:].any()
+    assert (img[:offset] == 7).all() and (img[offset + n:] == 9).all()
