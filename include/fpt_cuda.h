@@ -959,7 +959,7 @@ struct FptCudaBatchStats {
     uint32_t kernel_launches_per_pass;
     uint32_t block_size;         /* march kernel */
     uint32_t registers;          /* march kernel registers per thread */
-    uint32_t wave_paths;         /* paths per wave */
+    uint32_t wave_paths;         /* paths per wave, over all formula groups */
     uint32_t tuned;              /* 1 when the autotuner's choice was used */
     uint64_t workload_key;
     uint32_t refill;             /* march finish/refill group (0: default 8) */

@@ -68,3 +68,31 @@ def test_batch_64_scenes_autotuned(native):
     assert st["tuned"] == 1 and st["workload_key"] == tune["workload_key"]
     assert st["paths"] == sum(b.cfg.width * b.cfg.height * 4 for b in bundles)
     assert st["elapsed_ms"] > 0
+
+
+def _of_kind(kind, k, width, height, bounces):
+    b = scenes.menger_plane(width, height, 2, seed=k) if kind == "menger" else scenes.mandelbulb_path(width, height, 2, bounces, seed=k)
+    if kind == "menger":
+        b.ext.sky_width = b.ext.sky_height = 0
+        b.cfg.render[0] = float(bounces)
+    elif kind == "box":
+        b = scenes.mandelbox_path(width, height, 2, bounces, seed=k)
+    elif kind == "bulb":
+        b.ext.power = 5.5
+    elif kind == "hybrid":
+        h = scenes.hybrid_ext()
+        for name in ("formula", "iterations", "menger_scale", "hybrid_period", "bailout"):
+            setattr(b.ext, name, getattr(h, name))
+    return b
+
+
+@pytest.mark.parametrize("kinds", [("box",), ("menger", "bulb8", "hybrid", "box", "bulb"), ("bulb", "box", "bulb", "box", "bulb8", "bulb")])
+def test_formula_groups_equal_scene_alone(native, kinds):
+    """Batches of one, of every and of interleaved formulas, with ragged sizes and uneven bounce counts: images come back
+    in the caller's order and equal, bit for bit, the scene's own batch."""
+    bundles = [_of_kind(kind, k + 1, 33 + 17 * k, 20 + 9 * ((k * 3) % 5), 1 + (k * 2) % 4) for k, kind in enumerate(kinds)]
+    lin, img, st = nx.render_batch(bundles, linear=True, rgba=True)
+    assert st["scenes"] == len(kinds) and st["graph_launches"] == 2
+    for k, b in enumerate(bundles):
+        alone, alone_img, _ = nx.render_batch([b], linear=True, rgba=True)
+        assert np.array_equal(lin[k], alone[0]) and np.array_equal(img[k], alone_img[0]), (k, kinds[k])
