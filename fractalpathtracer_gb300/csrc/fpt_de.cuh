@@ -459,6 +459,30 @@ template <class T> __device__ __forceinline__ void menger_step(T &x, T &y, T &z,
     dr = dr * T(s);
 }
 
+// The same step in FP32: the descending sort by minima and maxima (six
+// operations instead of three comparisons and six selections).  They propagate
+// not-a-number, so an orbit that holds one is still not finite.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void menger_step_f32(float &x, float &y, float &z, float &dr, float s) {
+    const float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
+    const float hi = max_nan(ax, az), lo = min_nan(ax, az), mid = max_nan(ay, lo);
+    const float o = s - 1.0f;
+    x = max_nan(hi, mid) * s - o;
+    y = min_nan(hi, mid) * s - o;
+    z = min_nan(ay, lo) * s;
+    if (z > 0.5f * o) z = z - o;
+    dr = dr * s;
+}
+
 // The orbit loop as start / step / finish (orbit_eval runs it to
 // completion).
 template <class T> struct Orbit {
@@ -630,7 +654,8 @@ __device__ __forceinline__ float orbit_iterate(Orbit<float> &o, const DeviceScen
         }
         r2 = sum_squares(o.x, o.y, o.z);
     } else {
-        orbit_formula<KIND>(o, S, o.i);
+        if (KIND == KIND_MENGER) menger_step_f32(o.x, o.y, o.z, o.dr, S.menger_scale);
+        else orbit_formula<KIND>(o, S, o.i);
         r2 = o.x * o.x + o.y * o.y + o.z * o.z;
     }
     ++o.i;

@@ -119,7 +119,7 @@ __device__ __forceinline__ bool march_update(March &m, const DeviceScene &S, flo
     float o = fabsf(d) * 0.99f;
     m.pos = m.pos + m.dir * o;
     float lod = m.min_dist;
-    if (m.lod_falloff > 0.00001f) {
+    if (m.lod_falloff > 0.00001f && S.render[5] != 0.0f) {   // a weight of 0 leaves the minimum distance
         float3 r = m.start - m.pos;
         float fog = dot(r, r);
         lod = mixf(lod, 0.1f, fog * m.lod_falloff);
