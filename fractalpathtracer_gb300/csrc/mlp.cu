@@ -12,13 +12,13 @@
 //                          features, activations, pre-activations and deltas
 //                          (bf16), and per warp its output-layer gradient and
 //                          loss sums
-//   wgrad_tc_kernel        tcgen05: per (layer, 512-row chunk of the batch)
+//   wgrad_tc_kernel        tcgen05: per (layer, 256-row chunk of the batch)
 //                          D = H^T dZ, a 128 x 64 FP32 accumulator in tensor
 //                          memory; a row of ones in H^T gives the bias
 //                          gradient in the same MMAs
-//   wgrad_reduce_kernel,   the chunks' and warps' partial sums added in a
-//   out_reduce_kernel      fixed order: gradients and loss are deterministic
-//   adam_kernel
+//   gradient_kernel        the chunks' and warps' partial sums added in a
+//                          fixed order (gradients and loss are deterministic),
+//                          and the Adam step
 // The skip march that uses the model is in skip.cuh (one instantiation per
 // scene kind).
 #include <cuda_bf16.h>
@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(32 * kWarpsTrain, 2) train_fwd_bwd_kernel(Trai
     float loss = valid ? wgt * e * e : 0.0f;
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     // output layer: dW4[j] = sum_b dout_b H4[b][j], db4 = sum_b dout_b; the warp's sums go to its
-    // partial row (out_reduce_kernel adds the warps in order)
+    // partial row (gradient_kernel adds the warps in a fixed order)
     float *part = A.out_part + size_t(blockIdx.x * kWarpsTrain + warp) * kOutPart;
     for (int j = 0; j < kHid; ++j) {
         float v = dout * __bfloat162float(h4[j]);
@@ -199,21 +200,41 @@ __global__ void __launch_bounds__(32 * kWarpsTrain, 2) train_fwd_bwd_kernel(Trai
 
 // ---------------------------------------------------------------- forward + backward on tcgen05
 // The training pass of train_fwd_bwd_kernel with its products on the
-// 5th-generation tensor cores: 128 rows per CTA, one row per thread, the
-// M = 128, N = 64, K = 16 MMA shape of the inference pass.  Forward: per
+// 5th-generation tensor cores: 128 rows per CTA, the M = 128, N = 64, K = 16
+// MMA shape of the inference pass, two threads per row (columns 0-31 and
+// 32-63: threads t and t + 128 read the same tensor-memory lane).  Forward: per
 // layer H_l x W_l^T into a 128 x 64 FP32 accumulator in tensor memory; each
-// thread reads its row, adds the bias, stores Z_l (bf16) and H_{l+1} =
-// SiLU(Z_l) (bf16) to global memory and into the next layer's operand tile.
-// Backward: dZ_4 = dout W4 o SiLU'(Z_4) per row, then dZ_l = (dZ_{l+1} W_l) o
-// SiLU'(Z_l) with B = W_l^T staged at set-up.  Same arithmetic as the
-// mma.sync pass (BF16 operands, FP32 accumulation, SiLU and its derivative on
-// the FP32 pre-activation / its bf16 copy); only the order of the FP32 sums
-// differs.
+// thread reads its half row, adds the bias, keeps Z_l (bf16) in registers for
+// the backward pass and writes H_{l+1} = SiLU(Z_l) (bf16) to global memory and
+// into the next layer's operand tile.  Backward: dZ_4 = dout W4 o SiLU'(Z_4)
+// per row, then dZ_l = (dZ_{l+1} W_l) o SiLU'(Z_l) with B = W_l^T staged at
+// set-up.  Same arithmetic as the mma.sync pass (BF16 operands, FP32
+// accumulation, SiLU and its derivative on the FP32 pre-activation / its bf16
+// copy); only the order of the FP32 sums differs.
+// Bound by latency: a 16384-row batch is 128 CTAs, one per SM, each a chain of
+// seven MMA rounds and their epilogues.  Hence the two threads per row, the
+// weights staged as 16-byte vectors (2-byte loads and stores before), the
+// 32 column sums of a warp in 31 shuffles (160 before) and one CTA barrier per
+// round: 43.3 -> 25.5 us per pass.
 // Two floats as a packed pair of bf16 (lo in the low half).
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     return uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(lo))) | (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << 16);
 }
+// Transposes an 8 x 8 block of 16-bit values: row r is in[r], out[c] is column c.
+__device__ __forceinline__ void transpose8(const uint4 in[8], uint4 out[8]) {
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(in);
+    uint32_t *o = reinterpret_cast<uint32_t *>(out);
+#pragma unroll
+    for (int p = 0; p < 4; ++p)   // columns 2p and 2p + 1: the halves of word p of each row
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            o[(2 * p) * 4 + r] = __byte_perm(w[(2 * r) * 4 + p], w[(2 * r + 1) * 4 + p], 0x5410);
+            o[(2 * p + 1) * 4 + r] = __byte_perm(w[(2 * r) * 4 + p], w[(2 * r + 1) * 4 + p], 0x7632);
+        }
+}
 
+constexpr int kTrainThreads = 2 * kTcRows;
+constexpr int kHalf = kHid / 2;   // columns per thread
 struct TrainTcSmem {
     alignas(128) unsigned char act[kTcRows * kInPad * 2];        // operand A: features, activations, then deltas
     alignas(128) unsigned char w0[kHid * kInPad * 2];            // forward B of layer 0: W0[n][k]
@@ -222,6 +243,7 @@ struct TrainTcSmem {
     float b[kHidden][kHid];
     float w4[kHid];
     float b4;
+    float out[kTcRows], dout[kTcRows];   // output layer: sums over columns 0-31, loss derivative
     uint32_t tmem;
     alignas(8) uint64_t bar;
     unsigned char slack[4096];
@@ -229,14 +251,14 @@ struct TrainTcSmem {
 inline size_t train_tc_smem_bytes() { return sizeof(TrainTcSmem); }
 
 // One round of MMAs (A = the act tile with K = k columns, B at `b`) into the
-// accumulator; every thread then holds its row in r.  False when the MMAs did
-// not complete within kMmaWaitNs (the same in every thread).
-__device__ __forceinline__ bool train_round(TrainTcSmem &sm, uint32_t b, int k, uint32_t &phase, uint32_t r[64]) {
+// accumulator; every thread then holds its half row in r.  `late`: this
+// thread's last wait ran out; false (the same in every thread) when any did.
+__device__ __forceinline__ bool train_round(TrainTcSmem &sm, uint32_t b, int k, uint32_t &phase, bool &late, uint32_t r[kHalf]) {
     const int t = threadIdx.x;
     const uint32_t act = umma::smem_u32(sm.act);
     umma::fence_smem_to_async();
     umma::fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(late)) return false;
     if (t == 0) {
         umma::fence_after_sync();
         for (int j = 0; j < k / 16; ++j)
@@ -244,39 +266,54 @@ __device__ __forceinline__ bool train_round(TrainTcSmem &sm, uint32_t b, int k, 
                            umma::smem_desc(b + uint32_t(j) * 2u * kWK, kWK, kCore), kTcIdesc, uint32_t(j));
         umma::mma_commit(&sm.bar);
     }
-    const int late = t == 0 ? int(!umma::mbar_wait(&sm.bar, phase, kMmaWaitNs)) : 0;
+    late = !umma::mbar_wait(&sm.bar, phase, kMmaWaitNs);
     phase ^= 1u;
-    if (__syncthreads_or(late)) return false;
     umma::fence_after_sync();
     __syncwarp();
-    umma::tmem_ld64(sm.tmem + (uint32_t(t & ~31) << 16), r);
+    umma::tmem_ld32(sm.tmem + (uint32_t(t & 96) << 16) + uint32_t(t >> 7) * kHalf, r);
     return true;
 }
 
-__device__ __forceinline__ void store_row64(__nv_bfloat16 *g, const uint32_t h[32]) {
+// A thread's 32 columns to global memory and, with `act`, into the operand tile.
+__device__ __forceinline__ void store_half_row(__nv_bfloat16 *g, const uint32_t h[kHalf / 2]) {
     uint4 *d = reinterpret_cast<uint4 *>(g);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) d[q] = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+    for (int q = 0; q < kHalf / 8; ++q) d[q] = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+}
+__device__ __forceinline__ void stage_half_row(uint32_t act, int row, int half, const uint32_t h[kHalf / 2]) {
+#pragma unroll
+    for (int q = 0; q < kHalf / 8; ++q)
+        umma::st_shared_v4(act + act_offset(row, half * (kHalf / 8) + q), h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
 }
 
-__global__ void __launch_bounds__(kTcRows) train_fwd_bwd_tc_kernel(TrainArgs A) {
+__global__ void __launch_bounds__(kTrainThreads) train_fwd_bwd_tc_kernel(TrainArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainTcSmem &sm = *reinterpret_cast<TrainTcSmem *>(smem_raw);
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, half = t >> 7, trow = t & (kTcRows - 1), c0 = half * kHalf;
     const Model &M = A.model;
     if (__syncthreads_or(t == 0 && *reinterpret_cast<volatile uint32_t *>(A.fail) != 0u)) return;   // an earlier launch timed out
-    for (int i = t; i < kHid * kInPad; i += kTcRows) {
-        const int n = i / kInPad, k = i - n * kInPad;
-        *reinterpret_cast<__nv_bfloat16 *>(sm.w0 + w_core_offset(n, k)) = M.wbf[kW0 + i];
+    // Weight rows as 16-byte vectors of 8 K values; W_l^T block by block.
+    for (int i = t; i < kHid * (kInPad / 8); i += kTrainThreads) {
+        const int n = i % kHid, k = i / kHid * 8;
+        *reinterpret_cast<uint4 *>(sm.w0 + w_core_offset(n, k)) = *reinterpret_cast<const uint4 *>(M.wbf + kW0 + n * kInPad + k);
     }
+#pragma unroll
     for (int l = 1; l < kHidden; ++l)
-        for (int i = t; i < kHid * kHid; i += kTcRows) {
-            const int n = i / kHid, k = i - n * kHid;
-            *reinterpret_cast<__nv_bfloat16 *>(sm.w[l - 1] + w_core_offset(n, k)) = M.wbf[w_offset(l) + i];
-            *reinterpret_cast<__nv_bfloat16 *>(sm.wt[l - 1] + w_core_offset(k, n)) = M.wbf[w_offset(l) + i];
+        for (int i = t; i < kHid * (kHid / 8); i += kTrainThreads) {
+            const int n = i % kHid, k = i / kHid * 8;
+            *reinterpret_cast<uint4 *>(sm.w[l - 1] + w_core_offset(n, k)) = *reinterpret_cast<const uint4 *>(M.wbf + w_offset(l) + n * kHid + k);
         }
-    for (int i = t; i < kHidden * kHid; i += kTcRows) sm.b[i / kHid][i % kHid] = M.params[b_offset(i / kHid) + i % kHid];
-    for (int i = t; i < kHid; i += kTcRows) sm.w4[i] = __bfloat162float(M.wbf[kW4 + i]);
+    if (t < (kHidden - 1) * 64) {
+        const int l = 1 + t / 64, nb = (t / 8) % 8, kb = t % 8;
+        uint4 in[8], out[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) in[j] = *reinterpret_cast<const uint4 *>(M.wbf + w_offset(l) + (nb * 8 + j) * kHid + kb * 8);
+        transpose8(in, out);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) *reinterpret_cast<uint4 *>(sm.wt[l - 1] + w_core_offset(kb * 8 + e, nb * 8)) = out[e];
+    }
+    for (int i = t; i < kHidden * kHid; i += kTrainThreads) sm.b[i / kHid][i % kHid] = M.params[b_offset(i / kHid) + i % kHid];
+    if (t < kHid) sm.w4[t] = __bfloat162float(M.wbf[kW4 + t]);
     if (t == 0) {
         sm.b4 = M.params[kB4];
         umma::mbar_init(&sm.bar, 1u);
@@ -290,108 +327,124 @@ __global__ void __launch_bounds__(kTcRows) train_fwd_bwd_tc_kernel(TrainArgs A) 
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t act = umma::smem_u32(sm.act);
-    const uint32_t row = blockIdx.x * kTcRows + uint32_t(t);
+    const uint32_t row = blockIdx.x * kTcRows + uint32_t(trow);
     const bool valid = row < A.batch;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     if (valid) s = A.data[A.identity ? row : hash2(A.seed + A.step * 7919u, row) % A.n_data];
     {
         const float u[3] = {(s.x - M.center[0]) * M.inv_half[0], (s.y - M.center[1]) * M.inv_half[1], (s.z - M.center[2]) * M.inv_half[2]};
-        uint32_t f[kInPad / 2];
-        feature_pairs(u, f);
-#pragma unroll
-        for (int kc = 0; kc < kInPad / 8; ++kc) umma::st_shared_v4(act + act_offset(t, kc), f[4 * kc], f[4 * kc + 1], f[4 * kc + 2], f[4 * kc + 3]);
         uint4 *gx = reinterpret_cast<uint4 *>(A.gx + size_t(row) * kInPad);
+        // Each half writes 7 of the 14 vectors (and the compiler drops the other features of its branch).
+        auto write_features = [&](auto first) {
+            uint32_t f[kInPad / 2];
+            feature_pairs(u, f);
 #pragma unroll
-        for (int q = 0; q < kInPad / 8; ++q) gx[q] = make_uint4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+            for (int q = 0; q < kInPad / 16; ++q) {
+                const int kc = decltype(first)::value + q;
+                umma::st_shared_v4(act + act_offset(trow, kc), f[4 * kc], f[4 * kc + 1], f[4 * kc + 2], f[4 * kc + 3]);
+                gx[kc] = make_uint4(f[4 * kc], f[4 * kc + 1], f[4 * kc + 2], f[4 * kc + 3]);
+            }
+        };
+        if (half == 0) write_features(std::integral_constant<int, 0>());
+        else write_features(std::integral_constant<int, kInPad / 16>());
     }
-    uint32_t phase = 0, r[64], h[32];
-    bool ok = true;
+    uint32_t phase = 0, r[kHalf], h[kHalf / 2], z[kHidden - 1][kHalf / 2];
+    bool ok = true, late = false;
     float dout = 0.0f, loss = 0.0f;
     // forward
-    for (int L = 0; L < kHidden && ok; ++L) {
-        ok = train_round(sm, umma::smem_u32(L == 0 ? sm.w0 : sm.w[L - 1]), L == 0 ? kInPad : kHid, phase, r);
-        if (!ok) break;
-        uint32_t z[32];
 #pragma unroll
-        for (int c = 0; c < kHid; c += 2) {
-            const float z0 = __uint_as_float(r[c]) + sm.b[L][c], z1 = __uint_as_float(r[c + 1]) + sm.b[L][c + 1];
-            z[c >> 1] = bf16_pair(z0, z1);
+    for (int L = 0; L < kHidden; ++L) {
+        if (ok) ok = train_round(sm, umma::smem_u32(L == 0 ? sm.w0 : sm.w[L > 0 ? L - 1 : 0]), L == 0 ? kInPad : kHid, phase, late, r);
+        if (!ok) break;
+#pragma unroll
+        for (int c = 0; c < kHalf; c += 2) {
+            const float z0 = __uint_as_float(r[c]) + sm.b[L][c0 + c], z1 = __uint_as_float(r[c + 1]) + sm.b[L][c0 + c + 1];
+            if (L + 1 < kHidden) z[L < kHidden - 1 ? L : 0][c >> 1] = bf16_pair(z0, z1);
             h[c >> 1] = bf16_pair(silu(z0), silu(z1));
         }
-        store_row64(A.gz[L] + size_t(row) * kHid, z);
         if (L + 1 < kHidden) {
-            store_row64(A.gh[L] + size_t(row) * kHid, h);
-#pragma unroll
-            for (int kc = 0; kc < kHid / 8; ++kc) umma::st_shared_v4(act + act_offset(t, kc), h[4 * kc], h[4 * kc + 1], h[4 * kc + 2], h[4 * kc + 3]);
+            store_half_row(A.gh[L < kHidden - 1 ? L : 0] + size_t(row) * kHid + c0, h);
+            stage_half_row(act, trow, half, h);
         }
     }
     if (ok) {
-        // output layer, loss, dZ4 (h holds H4, r + bias the FP32 Z4)
+        // output layer, loss, dZ4 (h holds H4, r + bias the FP32 Z4); the sum runs over the columns in order, so the
+        // second half of a row goes on from the first's
         float out = sm.b4;
+        auto add_columns = [&]() {
 #pragma unroll
-        for (int c = 0; c < kHid; c += 2) {
-            out += __uint_as_float(h[c >> 1] << 16) * sm.w4[c];
-            out += __uint_as_float(h[c >> 1] & 0xffff0000u) * sm.w4[c + 1];
-        }
-        const float y = s.w * A.inv_label_scale;
-        const float e = out - y;
-        const float wgt = e > 0.0f ? A.over_weight : 1.0f;
-        dout = valid ? 2.0f * wgt * e / float(A.batch) : 0.0f;
-        loss = valid ? wgt * e * e : 0.0f;
-        float *part = A.out_part + size_t(blockIdx.x * (kTcRows / 32) + warp) * kOutPart;
-        for (int c = 0; c < kHid; ++c) {
-            const uint32_t hb = (c & 1) ? (h[c >> 1] & 0xffff0000u) : (h[c >> 1] << 16);
-            float v = dout * __uint_as_float(hb);
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) part[c] = v;
-        }
-        {
-            float v = dout, lv = loss;
-            for (int o = 16; o > 0; o >>= 1) {
-                v += __shfl_xor_sync(0xffffffffu, v, o);
-                lv += __shfl_xor_sync(0xffffffffu, lv, o);
+            for (int c = 0; c < kHalf; c += 2) {
+                out += __uint_as_float(h[c >> 1] << 16) * sm.w4[c0 + c];
+                out += __uint_as_float(h[c >> 1] & 0xffff0000u) * sm.w4[c0 + c + 1];
             }
-            if (lane == 0) {
-                part[kHid] = v;
-                part[kHid + 1] = lv;
+        };
+        if (half == 0) {
+            add_columns();
+            sm.out[trow] = out;
+        }
+        __syncthreads();
+        if (half == 1) {
+            out = sm.out[trow];
+            add_columns();
+            const float y = s.w * A.inv_label_scale;
+            const float e = out - y;
+            const float wgt = e > 0.0f ? A.over_weight : 1.0f;
+            dout = valid ? 2.0f * wgt * e / float(A.batch) : 0.0f;
+            loss = valid ? wgt * e * e : 0.0f;
+            sm.dout[trow] = dout;
+        }
+        __syncthreads();
+        dout = sm.dout[trow];
+        // The warp's sums over its 32 rows: of dout (first half) or the loss (second) and of each of the 32 columns.
+        // Pairs of rows 16, 8, 4, 2, 1 apart are added in turn; a lane that adds for some columns hands its value
+        // of the others over, and ends with column `lane`.
+        float *part = A.out_part + size_t(blockIdx.x * (kTcRows / 32) + (trow >> 5)) * kOutPart;
+        float v = half == 0 ? dout : loss;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) part[kHid + half] = v;
+        float col[kHalf];
+#pragma unroll
+        for (int c = 0; c < kHalf; c += 2) {
+            col[c] = dout * __uint_as_float(h[c >> 1] << 16);
+            col[c + 1] = dout * __uint_as_float(h[c >> 1] & 0xffff0000u);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int c = 0; c < o; ++c) {
+                const float keep = upper ? col[c + o] : col[c], give = upper ? col[c] : col[c + o];
+                col[c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
         }
-        uint32_t d[32];
+        part[c0 + lane] = col[0];
+        uint32_t d[kHalf / 2];
 #pragma unroll
-        for (int c = 0; c < kHid; c += 2) {
-            const float z0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c]) + sm.b[3][c]));
-            const float z1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c + 1]) + sm.b[3][c + 1]));
-            d[c >> 1] = bf16_pair(dout * sm.w4[c] * silu_grad(z0), dout * sm.w4[c + 1] * silu_grad(z1));
+        for (int c = 0; c < kHalf; c += 2) {
+            const float z0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c]) + sm.b[3][c0 + c]));
+            const float z1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[c + 1]) + sm.b[3][c0 + c + 1]));
+            d[c >> 1] = bf16_pair(dout * sm.w4[c0 + c] * silu_grad(z0), dout * sm.w4[c0 + c + 1] * silu_grad(z1));
         }
-        store_row64(A.gdz[3] + size_t(row) * kHid, d);
-#pragma unroll
-        for (int kc = 0; kc < kHid / 8; ++kc) umma::st_shared_v4(act + act_offset(t, kc), d[4 * kc], d[4 * kc + 1], d[4 * kc + 2], d[4 * kc + 3]);
+        store_half_row(A.gdz[3] + size_t(row) * kHid + c0, d);
+        stage_half_row(act, trow, half, d);
     }
     // backward through hidden layers 3, 2, 1: dZ_l = (dZ_{l+1} W_l) o SiLU'(Z_l)
-    for (int l = kHidden - 1; l >= 1 && ok; --l) {
-        ok = train_round(sm, umma::smem_u32(sm.wt[l - 1]), kHid, phase, r);
+#pragma unroll
+    for (int l = kHidden - 1; l >= 1; --l) {
+        if (ok) ok = train_round(sm, umma::smem_u32(sm.wt[l - 1]), kHid, phase, late, r);
         if (!ok) break;
-        const uint4 *zg = reinterpret_cast<const uint4 *>(A.gz[l - 1] + size_t(row) * kHid);
-        uint32_t d[32];
+        uint32_t d[kHalf / 2];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const uint4 zz = zg[q];
-            const uint32_t zw[4] = {zz.x, zz.y, zz.z, zz.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int c = q * 8 + e * 2;
-                const float z0 = __uint_as_float(zw[e] << 16), z1 = __uint_as_float(zw[e] & 0xffff0000u);
-                d[c >> 1] = bf16_pair(__uint_as_float(r[c]) * silu_grad(z0), __uint_as_float(r[c + 1]) * silu_grad(z1));
-            }
+        for (int c = 0; c < kHalf; c += 2) {
+            const uint32_t zw = z[l - 1][c >> 1];
+            const float z0 = __uint_as_float(zw << 16), z1 = __uint_as_float(zw & 0xffff0000u);
+            d[c >> 1] = bf16_pair(__uint_as_float(r[c]) * silu_grad(z0), __uint_as_float(r[c + 1]) * silu_grad(z1));
         }
-        store_row64(A.gdz[l - 1] + size_t(row) * kHid, d);
-        if (l > 1) {
-#pragma unroll
-            for (int kc = 0; kc < kHid / 8; ++kc) umma::st_shared_v4(act + act_offset(t, kc), d[4 * kc], d[4 * kc + 1], d[4 * kc + 2], d[4 * kc + 3]);
-        }
+        store_half_row(A.gdz[l - 1] + size_t(row) * kHid + c0, d);
+        if (l > 1) stage_half_row(act, trow, half, d);
     }
     umma::fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(late)) ok = false;
     if (t < 32) {
         __syncwarp();
         umma::fence_after_sync();
@@ -406,74 +459,72 @@ __global__ void __launch_bounds__(kTcRows) train_fwd_bwd_tc_kernel(TrainArgs A) 
 // bias gradient db_l[n]).  A = H^T (128 x 64-row tile of the batch, K-major),
 // B = dZ^T (64 x 64), the M = 128, N = 64, K = 16 MMA shape of the forward
 // pass, accumulated over the chunk in one 64-column tensor-memory tile.  Each
-// CTA writes its 128 x 64 partial; wgrad_reduce_kernel adds the chunks in
+// CTA writes its partial as [n][m]; gradient_kernel adds the chunks in
 // order (no atomics: the same data gives the same bits).
+// Bound by latency (four rounds of loads, transpose and MMAs).  The tiles are
+// transposed in registers, 8 x 8 values at a time, and stored as 16-byte
+// vectors; core matrices lie 144 bytes apart instead of 128, so that the
+// vectors of 8 neighbouring blocks fall into different banks: 25.6 -> 10.9 us for
+// a 16384-row batch.
 constexpr uint32_t kWgChunk = 256;            // batch rows per CTA
 constexpr uint32_t kWgTile = 64;              // batch rows per round of 4 MMAs
+constexpr uint32_t kWgCore = kCore + 16;      // distance of core matrices along M / N
+constexpr uint32_t kWgAK = (kTcRows / 8) * kWgCore, kWgBK = (kHid / 8) * kWgCore;   // along K (batch rows)
 struct WgSmem {
-    alignas(128) unsigned char a[kTcRows * kWgTile * 2];   // H^T tile, [k chunk][m group][8 m][8 k]
-    alignas(128) unsigned char b[kHid * kWgTile * 2];      // dZ^T tile, [k chunk][n group][8 n][8 k]
+    alignas(128) unsigned char a[kWgAK * (kWgTile / 8)];   // H^T tile, [k chunk][m group][8 m][8 k]
+    alignas(128) unsigned char b[kWgBK * (kWgTile / 8)];   // dZ^T tile, [k chunk][n group][8 n][8 k]
     uint32_t tmem;
     alignas(8) uint64_t bar;
     unsigned char slack[4096];                             // keeps descriptor reads inside the CTA's shared memory
 };
 inline size_t wgrad_smem_bytes() { return sizeof(WgSmem); }
+__device__ __forceinline__ uint32_t wg_a_offset(int m, int kc) { return uint32_t(kc) * kWgAK + uint32_t(m >> 3) * kWgCore + uint32_t(m & 7) * 16u; }
+__device__ __forceinline__ uint32_t wg_b_offset(int n, int kc) { return uint32_t(kc) * kWgBK + uint32_t(n >> 3) * kWgCore + uint32_t(n & 7) * 16u; }
 
 struct WgradArgs {
     const __nv_bfloat16 *h[kHidden];     // H_0 = features (kInPad columns), H_1..H_3 (kHid columns)
     const __nv_bfloat16 *dz[kHidden];    // dZ_1..dZ_4 (kHid columns)
     uint32_t batch, chunks;
-    float *part;                         // [layer][chunk][128][64] partial sums
+    float *part;                         // [layer][chunk][64 n][128 m] partial sums (m <= K_l written)
     uint32_t *fail;                      // set (bit 2) when an MMA does not complete in time; later launches skip their work
 };
 
-// Global tile loads of one round (64 batch rows): H rows as 16-byte vectors
-// (8 columns each, at most 7 per thread) and dZ rows (4 per thread).
+// The 8 x 8 blocks of one round (64 batch rows): H has kcols / 8 x 8 of them, dZ 64; block i of the two together is
+// thread i's (and i - 128's, for layer 0).
 struct WgLoad {
-    uint4 h[(kTcRows * kWgTile / 8 + kTcRows - 1) / kTcRows];
-    uint4 dz[kHid * kWgTile / 8 / kTcRows];
+    uint4 v[2][8];
 };
 __device__ __forceinline__ void wg_load(WgLoad &L, const __nv_bfloat16 *H, const __nv_bfloat16 *DZ, int kcols, uint32_t kb, uint32_t b1) {
-    const int t = threadIdx.x, nvec = kcols / 8;
+    const int hcols = kcols / 8, hblocks = hcols * 8;
 #pragma unroll
-    for (int q = 0; q < int(sizeof(L.h) / sizeof(uint4)); ++q) {
-        const int i = t + q * kTcRows, row = i / nvec, v = i - row * nvec;
-        L.h[q] = (row < int(kWgTile) && kb + uint32_t(row) < b1)
-                     ? *reinterpret_cast<const uint4 *>(H + size_t(kb + row) * kcols + v * 8)
-                     : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int q = 0; q < int(sizeof(L.dz) / sizeof(uint4)); ++q) {
-        const int i = t + q * kTcRows, row = i >> 3, v = i & 7;
-        L.dz[q] = kb + uint32_t(row) < b1 ? *reinterpret_cast<const uint4 *>(DZ + size_t(kb + row) * kHid + v * 8)
-                                          : make_uint4(0u, 0u, 0u, 0u);
-    }
-}
-// The loaded vectors into the K-major operand tiles (a transpose: each of a
-// vector's 8 values goes to its own row of H^T / dZ^T), and the row of ones.
-__device__ __forceinline__ void wg_store(const WgLoad &L, WgSmem &sm, int kcols, uint32_t kb, uint32_t b1) {
-    const int t = threadIdx.x, nvec = kcols / 8;
-#pragma unroll
-    for (int q = 0; q < int(sizeof(L.h) / sizeof(uint4)); ++q) {
-        const int i = t + q * kTcRows, row = i / nvec, v = i - row * nvec;
-        if (row >= int(kWgTile)) continue;
-        const uint32_t w[4] = {L.h[q].x, L.h[q].y, L.h[q].z, L.h[q].w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int m = v * 8 + e;
-            *reinterpret_cast<uint16_t *>(sm.a + act_offset(m, row >> 3) + (row & 7) * 2) = uint16_t(w[e >> 1] >> ((e & 1) * 16));
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < int(sizeof(L.dz) / sizeof(uint4)); ++q) {
-        const int i = t + q * kTcRows, row = i >> 3, v = i & 7;
-        const uint32_t w[4] = {L.dz[q].x, L.dz[q].y, L.dz[q].z, L.dz[q].w};
+    for (int q = 0; q < 2; ++q) {
+        const int i = int(threadIdx.x) + q * kTcRows;
+        if (i >= hblocks + 64) break;
+        const bool dz = i >= hblocks;
+        const int cols = dz ? 8 : hcols, j = dz ? i - hblocks : i, rb = j / cols, cb = j - rb * cols;
+        const __nv_bfloat16 *src = (dz ? DZ : H) + size_t(kb + uint32_t(rb) * 8u) * (cols * 8) + cb * 8;
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            *reinterpret_cast<uint16_t *>(sm.b + w_core_offset(v * 8 + e, row)) = uint16_t(w[e >> 1] >> ((e & 1) * 16));
+            L.v[q][e] = kb + uint32_t(rb * 8 + e) < b1 ? *reinterpret_cast<const uint4 *>(src + size_t(e) * (cols * 8)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+// The loaded blocks, transposed, into the K-major operand tiles, and the row of ones.
+__device__ __forceinline__ void wg_store(const WgLoad &L, WgSmem &sm, int kcols, uint32_t kb, uint32_t b1) {
+    const int t = threadIdx.x, hcols = kcols / 8, hblocks = hcols * 8;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int i = t + q * kTcRows;
+        if (i >= hblocks + 64) break;
+        const bool dz = i >= hblocks;
+        const int cols = dz ? 8 : hcols, j = dz ? i - hblocks : i, rb = j / cols, cb = j - rb * cols;
+        uint4 out[8];
+        transpose8(L.v[q], out);
+        unsigned char *dst = dz ? sm.b + wg_b_offset(cb * 8, rb) : sm.a + wg_a_offset(cb * 8, rb);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) *reinterpret_cast<uint4 *>(dst + e * 16) = out[e];
     }
     if (t < int(kWgTile))   // H^T row kcols: ones on the chunk's rows, so its product with dZ is the bias gradient
-        *reinterpret_cast<uint16_t *>(sm.a + act_offset(kcols, t >> 3) + (t & 7) * 2) = kb + uint32_t(t) < b1 ? 0x3F80u : 0u;
+        *reinterpret_cast<uint16_t *>(sm.a + wg_a_offset(kcols, t >> 3) + (t & 7) * 2) = kb + uint32_t(t) < b1 ? 0x3F80u : 0u;
 }
 
 __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
@@ -483,10 +534,10 @@ __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
     const int layer = blockIdx.y;
     const int kcols = layer == 0 ? kInPad : kHid;
     const __nv_bfloat16 *H = G.h[layer], *DZ = G.dz[layer];
-    float *out = G.part + ((size_t(layer) * G.chunks + blockIdx.x) * kTcRows + uint32_t(t)) * kHid;
+    float *out = G.part + (size_t(layer) * G.chunks + blockIdx.x) * (kTcRows * kHid) + uint32_t(t);
     // an earlier launch gave up: no MMA here (one read, the same decision in every thread)
     if (__syncthreads_or(t == 0 && *reinterpret_cast<volatile uint32_t *>(G.fail) != 0u)) {
-        for (int n = 0; n < kHid; ++n) out[n] = 0.0f;
+        for (int n = 0; n < kHid && t <= kcols; ++n) out[n * kTcRows] = 0.0f;
         return;
     }
     if (t == 0) umma::mbar_init(&sm.bar, 1u);
@@ -496,10 +547,8 @@ __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
         umma::tmem_relinquish();
     }
     // H^T rows above the ones row stay zero for every round
-    for (int i = t; i < (kTcRows - kcols - 1) * int(kWgTile); i += kTcRows) {
-        const int m = kcols + 1 + i / int(kWgTile), k = i % int(kWgTile);
-        *reinterpret_cast<uint16_t *>(sm.a + act_offset(m, k >> 3) + (k & 7) * 2) = 0u;
-    }
+    for (int i = t; i < (kTcRows - kcols - 1) * int(kWgTile / 8); i += kTcRows)
+        *reinterpret_cast<uint4 *>(sm.a + wg_a_offset(kcols + 1 + i / int(kWgTile / 8), i % int(kWgTile / 8))) = make_uint4(0u, 0u, 0u, 0u);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -518,7 +567,7 @@ __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
             umma::fence_after_sync();
 #pragma unroll
             for (uint32_t j = 0; j < kWgTile / 16; ++j)
-                umma::mma_bf16(sm.tmem, umma::smem_desc(a + j * 2u * kActK, kActK, kCore), umma::smem_desc(bt + j * 2u * kWK, kWK, kCore),
+                umma::mma_bf16(sm.tmem, umma::smem_desc(a + j * 2u * kWgAK, kWgAK, kWgCore), umma::smem_desc(bt + j * 2u * kWgBK, kWgBK, kWgCore),
                                kTcIdesc, (any || j > 0u) ? 1u : 0u);
             umma::mma_commit(&sm.bar);
         }
@@ -536,12 +585,12 @@ __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
         __syncwarp();
         uint32_t r[64];
         umma::tmem_ld64(sm.tmem + (uint32_t(t & ~31) << 16), r);
+        if (t <= kcols) {
 #pragma unroll
-        for (int n = 0; n < kHid; n += 4)
-            *reinterpret_cast<float4 *>(out + n) = make_float4(__uint_as_float(r[n]), __uint_as_float(r[n + 1]), __uint_as_float(r[n + 2]),
-                                                               __uint_as_float(r[n + 3]));
+            for (int n = 0; n < kHid; ++n) out[n * kTcRows] = __uint_as_float(r[n]);
+        }
     } else {
-        for (int n = 0; n < kHid; ++n) out[n] = 0.0f;
+        for (int n = 0; n < kHid && t <= kcols; ++n) out[n * kTcRows] = 0.0f;
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -553,54 +602,67 @@ __global__ void __launch_bounds__(kTcRows) wgrad_tc_kernel(WgradArgs G) {
     if (fail && t == 0) atomicOr(G.fail, 2u);
 }
 
-// grad += the chunks' partials, added in chunk order: one thread per (layer, m <= K_l, n).
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *part, uint32_t chunks, float *grad) {
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= uint32_t(kHidden) * kTcRows * kHid) return;
-    const int layer = int(idx / (kTcRows * kHid)), m = int((idx / kHid) % kTcRows), n = int(idx % kHid);
-    const int kcols = k_of(layer);
-    if (m > kcols) return;
-    float s = 0.0f;
-    for (uint32_t c = 0; c < chunks; ++c) s += part[((size_t(layer) * chunks + c) * kTcRows + m) * kHid + n];
-    if (m < kcols) grad[w_offset(layer) + n * kcols + m] += s;
-    else grad[b_offset(layer) + n] += s;
+// ---------------------------------------------------------------- gradient sums and Adam
+// Adds the partial sums of a pass in a fixed order.  A block of the first
+// kHidden x 64 has row n of one layer: thread m adds the chunks of weight
+// (n, m) in order, thread K_l those of the bias.  The other blocks have 8
+// columns each of the output layer and the loss: thread (j, g) adds warps g,
+// g + 8, ... in order, and the 8 group sums are added in order.
+// ADAM: the sum goes straight into the parameter's Adam step; otherwise it is
+// added to the gradient vector.  (Reduction, output reduction and Adam were
+// three launches, the output reduction one block: 16.5 -> 8.7 us.)
+constexpr int kOutGroups = 8, kOutCols = 8;
+constexpr uint32_t kSumBlocks = kHidden * kHid + (kOutPart + kOutCols - 1) / kOutCols;
+struct SumArgs {
+    const float *w_part, *out_part;
+    uint32_t chunks, warps;
+    float *grad;          // !ADAM: kParams gradients, accumulated
+    float *loss;          // accumulated
+    float *params, *m, *v;   // ADAM: parameters and moments
+    __nv_bfloat16 *wbf;
+    float lr, b1t, b2t;
+};
+__device__ __forceinline__ void adam_step(const SumArgs &S, int i, float g) {
+    const float mi = 0.9f * S.m[i] + 0.1f * g;
+    const float vi = 0.999f * S.v[i] + 0.001f * g * g;
+    S.m[i] = mi;
+    S.v[i] = vi;
+    float p = S.params[i];
+    p -= S.lr * (mi / (1.0f - S.b1t)) / (sqrtf(vi / (1.0f - S.b2t)) + 1e-8f);
+    S.params[i] = p;
+    S.wbf[i] = __float2bfloat16_rn(p);
 }
-
-// Output layer and loss: grad[W4], grad[b4] and the loss += the warps' partial
-// sums.  Thread (j, g) adds warps g, g + 8, ... in order; thread (j, 0) then
-// adds the 8 group sums in order (a fixed order: the same bits every run).
-constexpr int kOutGroups = 8;
-__global__ void __launch_bounds__(kOutPart * kOutGroups) out_reduce_kernel(const float *part, uint32_t warps, float *grad, float *loss) {
-    __shared__ float sums[kOutGroups][kOutPart];
-    const uint32_t j = threadIdx.x % kOutPart, g = threadIdx.x / kOutPart;
-    float s = 0.0f;
-    for (uint32_t w = g; w < warps; w += kOutGroups) s += part[size_t(w) * kOutPart + j];
-    sums[g][j] = s;
+template <bool ADAM> __global__ void __launch_bounds__(kTcRows) gradient_kernel(SumArgs S) {
+    const int t = threadIdx.x;
+    if (blockIdx.x < uint32_t(kHidden * kHid)) {
+        const int layer = int(blockIdx.x) / kHid, n = int(blockIdx.x) % kHid, kcols = k_of(layer);
+        if (t > kcols) return;
+        const float *part = S.w_part + (size_t(layer) * S.chunks * kHid + n) * kTcRows + t;
+        float s = 0.0f;
+#pragma unroll 16
+        for (uint32_t c = 0; c < S.chunks; ++c) s += part[size_t(c) * (kHid * kTcRows)];
+        const int i = t < kcols ? w_offset(layer) + n * kcols + t : b_offset(layer) + n;
+        if (!ADAM) S.grad[i] += s;
+        else if (!(layer == 0 && t >= kIn && t < kInPad)) adam_step(S, i, 0.0f + s);   // padded feature columns of W0 stay zero
+        return;
+    }
+    __shared__ float sums[kOutGroups][kOutCols];
+    const int j = int(blockIdx.x - uint32_t(kHidden * kHid)) * kOutCols + t % kOutCols, g = t / kOutCols;
+    const bool mine = g < kOutGroups && j < int(kOutPart);
+    if (mine) {
+        float s = 0.0f;
+#pragma unroll 16
+        for (uint32_t w = uint32_t(g); w < S.warps; w += kOutGroups) s += S.out_part[size_t(w) * kOutPart + j];
+        sums[g][t % kOutCols] = s;
+    }
     __syncthreads();
-    if (g != 0u) return;
+    if (!mine || g != 0) return;
     float total = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kOutGroups; ++k) total += sums[k][j];
-    if (j < uint32_t(kHid)) grad[kW4 + j] += total;
-    else if (j == uint32_t(kHid)) grad[kB4] += total;
-    else *loss += total;
-}
-
-__global__ void __launch_bounds__(256) adam_kernel(float *params, float *m, float *v, float *grad, __nv_bfloat16 *wbf, float lr,
-                                                   float b1t, float b2t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
-    const bool pad = i < kB0 && (i % kInPad) >= kIn;   // padded feature columns of W0 stay zero
-    const float g = pad ? 0.0f : grad[i];
-    const float mi = 0.9f * m[i] + 0.1f * g;
-    const float vi = 0.999f * v[i] + 0.001f * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float p = params[i];
-    if (!pad) p -= lr * (mi / (1.0f - b1t)) / (sqrtf(vi / (1.0f - b2t)) + 1e-8f);
-    params[i] = p;
-    wbf[i] = __float2bfloat16_rn(p);
-    grad[i] = 0.0f;
+    for (int k = 0; k < kOutGroups; ++k) total += sums[k][t];
+    if (j == kHid + 1) *S.loss += total;
+    else if (!ADAM) S.grad[j < kHid ? kW4 + j : kB4] += total;
+    else adam_step(S, j < kHid ? kW4 + j : kB4, 0.0f + total);
 }
 
 __global__ void to_bf16_kernel(const float *params, __nv_bfloat16 *wbf) {
@@ -809,13 +871,14 @@ static void set_attributes() {
     done = true;
 }
 
-// Forward + backward of one batch: accumulates into A.grad and A.loss.
-static void launch_gradients(const TrainArgs &A, cudaStream_t st) {
+// Forward + backward of one batch: accumulates into A.grad and A.loss, or, with `adam` (its parameters, moments and
+// step), takes the Adam step and accumulates the loss.
+static void launch_gradients(const TrainArgs &A, const SumArgs *adam, cudaStream_t st) {
     set_attributes();
     const uint32_t blocks = (A.batch + kRowsPerBlock - 1) / kRowsPerBlock;
     // forward + backward on the network engine of the inference passes (tcgen05 by default)
     if (ctx().network_engine == FPT_CUDA_NET_MMA_SYNC) train_fwd_bwd_kernel<<<blocks, 32 * kWarpsTrain, train_smem_bytes(), st>>>(A);
-    else train_fwd_bwd_tc_kernel<<<blocks, kTcRows, train_tc_smem_bytes(), st>>>(A);
+    else train_fwd_bwd_tc_kernel<<<blocks, kTrainThreads, train_tc_smem_bytes(), st>>>(A);
     WgradArgs G;
     G.h[0] = A.gx;
     for (int l = 1; l < kHidden; ++l) G.h[l] = A.gh[l - 1];
@@ -825,8 +888,15 @@ static void launch_gradients(const TrainArgs &A, cudaStream_t st) {
     G.part = A.w_part;
     G.fail = A.fail;
     wgrad_tc_kernel<<<dim3(G.chunks, kHidden), kTcRows, wgrad_smem_bytes(), st>>>(G);
-    wgrad_reduce_kernel<<<(kHidden * kTcRows * kHid + 255) / 256, 256, 0, st>>>(A.w_part, G.chunks, A.grad);
-    out_reduce_kernel<<<1, kOutPart * kOutGroups, 0, st>>>(A.out_part, blocks * kWarpsTrain, A.grad, A.loss);
+    SumArgs S = adam ? *adam : SumArgs{};
+    S.w_part = A.w_part;
+    S.out_part = A.out_part;
+    S.chunks = G.chunks;
+    S.warps = blocks * kWarpsTrain;
+    S.grad = A.grad;
+    S.loss = A.loss;
+    if (adam) gradient_kernel<true><<<kSumBlocks, kTcRows, 0, st>>>(S);
+    else gradient_kernel<false><<<kSumBlocks, kTcRows, 0, st>>>(S);
 }
 
 static HostModel *find(uint64_t id) {
@@ -994,11 +1064,13 @@ int fpt_cuda_mlp_create(const struct FptRenderConfig *config, const struct FptCu
             mlp::TrainArgs A;
             mlp::fill_train_args(A, *hm, hm->data, hm->n_data, mc->batch, over);
             A.seed = seed;
-            mlp::launch_gradients(A, c.stream);
             hm->step += 1;
             const float lr = std::max(lr0 * 0.5f * (1.0f + std::cos(3.14159265f * float(s) / float(mc->steps))), lr0 * 0.02f);
             const float b1t = std::pow(0.9f, float(hm->step)), b2t = std::pow(0.999f, float(hm->step));
-            mlp::adam_kernel<<<(mlp::kParams + 255) / 256, 256, 0, c.stream>>>(hm->params, hm->m, hm->v, hm->grad, hm->wbf, lr, b1t, b2t);
+            mlp::SumArgs adam{};
+            adam.params = hm->params; adam.m = hm->m; adam.v = hm->v; adam.wbf = hm->wbf;
+            adam.lr = lr; adam.b1t = b1t; adam.b2t = b2t;
+            mlp::launch_gradients(A, &adam, c.stream);
             if (probe) {
                 float l = 0.0f;
                 if (!check(cudaMemcpyAsync(&l, hm->loss, 4, cudaMemcpyDeviceToHost, c.stream), "loss readback", error, error_len) ||
@@ -1147,7 +1219,7 @@ int fpt_cuda_mlp_gradients(uint64_t model, const float *points_xyzw, size_t n, f
               check(cudaMemsetAsync(hm->grad, 0, mlp::kParams * 4, c.stream), "grad reset", error, error_len) &&
               check(cudaMemsetAsync(hm->loss, 0, 4, c.stream), "loss reset", error, error_len);
     if (!ok) return 1;
-    mlp::launch_gradients(A, c.stream);
+    mlp::launch_gradients(A, nullptr, c.stream);
     float l = 0.0f;
     ok = check(cudaGetLastError(), "gradient launch", error, error_len) &&
          check(cudaMemcpyAsync(gradients, hm->grad, mlp::kParams * 4, cudaMemcpyDeviceToHost, c.stream), "gradient readback", error, error_len) &&
