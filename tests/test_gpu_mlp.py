@@ -112,6 +112,19 @@ def test_gradients_match_oracle(blank_model, engine):
     assert np.abs(pad).max() < 1e-3 * np.abs(g[:7168]).max()   # padding columns carry no real gradient
 
 
+@pytest.mark.parametrize("rows", [1, 8, 63, 65, 128, 129, 255, 257, 449])
+def test_gradient_tile_edges(blank_model, rows):
+    """Batches that end inside an 8-row block, a 64-row tile, a 128-row CTA and a 256-row chunk, against the oracle
+    (the tolerance of test_gradients_match_oracle, over the whole gradient)."""
+    params = scenes.random_mlp_params(14)
+    nx.mlp_set_params(blank_model, params)
+    pts = _points(rows, 9)
+    g, loss = nx.mlp_gradients(blank_model, pts, 10.0)
+    g_ref, loss_ref = oracle.mlp_gradients(params, *BULB_BOX, pts, 10.0, emulate_bf16=True)
+    assert abs(loss - loss_ref) <= 2e-2 * loss_ref
+    assert np.linalg.norm(g - g_ref) <= 2e-2 * np.linalg.norm(g_ref) + 1e-7
+
+
 def test_gradients_are_deterministic(blank_model):
     """The weight and bias gradients come from tcgen05 MMAs per 512-row chunk and a reduction in chunk order, the
     output layer and the loss from per-warp sums added in warp order: no floating-point atomics, so the same batch
