@@ -385,11 +385,16 @@ struct MarchJob {
     float3 rp0;         // shadow: hit point the ray leaves
 };
 
+// Resident blocks per SM that the register allocation aims at: the Menger fold's
+// short steps are worth more warps (720p 16 spp: 7 blocks 15.6 ms, 8 15.2, 9
+// 14.8, 10 15.1), the others are not (Mandelbulb 1080p 16 spp 28.9 at 7 to 9,
+// Mandelbox 1080p 4 spp 12.4, 12.5, 13.0).
+template <int KIND> constexpr int kMarchBlocks = KIND == KIND_MENGER ? 9 : 7;
 // FP64: the camera-ray pass of a deep-zoom scene (FptCudaSceneExt.fp64_bisection,
 // a pinhole camera): a camera ray whose FP32 march stopped because a step no
 // longer moved its position (shaders/Shaders.metal:3726, 3739-3746) continues
 // in FP64 (march_fp64), which decides hit or miss and the hit distance.
-template <int KIND, bool BATCH = false, int BLOCK = 128, int MINB = 7, bool FP64 = false>
+template <int KIND, bool BATCH = false, int BLOCK = 128, int MINB = kMarchBlocks<KIND>, bool FP64 = false>
 __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cur) {
     const DeviceScene *sp = BATCH ? W.scene : &c_scene;   // the lane's scene (per job when BATCH)
     const uint32_t n_path = W.counters[C_MARCH0 + cur];
@@ -405,7 +410,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
     float box_exit = 3.0e38f;
     float known_d = 0.0f;            // exact distance at the march start handed over by the skip pass
     bool have_d = false;
-    bool active = false, pending = false, retired = false;
+    bool active = false, retired = false;
+    // The warp's lanes that still take rays, and those of them to refill.  A
+    // lane of `left` either marches or waits with a finished ray, so one vote per
+    // trip (who marches) tells everything else.
+    unsigned left = FULL, need = FULL;
+    const uint32_t refill_batch = W.refill_batch ? W.refill_batch : kRefillBatch;
     uint32_t c_primary = 0, c_secondary = 0, c_shadow = 0, c_paths = 0;
     // Profile counters kept off the registers of the march: orbit iterations of
     // the lane's current job in one register, block totals in shared memory
@@ -423,12 +433,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
     while (true) {
         if (loop_guard(trips, t0, W.counters, W.loop_limit_ns)) break;
         // Refill every lane whose march finished: one atomic per warp.
-        unsigned need = __ballot_sync(FULL, !active && !pending && !retired);
         if (need) {
             uint32_t leader = __ffs(need) - 1, base = 0;
             if (lane == leader) base = atomicAdd(&W.counters[C_HEAD], (unsigned)__popc(need));
             base = __shfl_sync(FULL, base, leader);
-            if (!active && !pending && !retired) {
+            if ((need >> lane) & 1u) {
                 uint32_t idx = base + __popc(need & ((1u << lane) - 1u));
                 if (idx >= total) {
                     retired = true;
@@ -469,7 +478,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
                         have_d = active && (st & PF_KNOWN_D);
                         known_d = R.grad.w;
                     }
-                    pending = !active;
                 } else {
                     const ShadowJob &J = qs[idx - n_path];
                     float4 o = J.origin, nn = J.normal, d = J.dir;
@@ -497,11 +505,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
                         have_d = active && d.w == 2.0f;
                         known_d = J.contrib.w;
                     }
-                    pending = !active;
                 }
             }
+            left = __ballot_sync(FULL, !retired);
+            need = 0u;
         }
-        if (!__any_sync(FULL, !retired)) break;
+        if (!left) break;
         const DeviceScene &S = *sp;
         TranslucencyProbe<KIND> probe{sp};
         // One distance evaluation for every lane with a march in flight.
@@ -517,22 +526,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
                 m.pos = job.shadow ? job.rp0 + m.dir * (S.render[4] * 1.01f + 1.0f)
                                    : m.pos + m.dir * (S.render[4] + len3(m.pos - cam) + 1.0f);
             }
-            pending = !active;
         }
         // Finished lanes write their results (and are refilled on the next
         // trip) together once `refill_batch` of them wait or nothing else runs:
         // the divergent finish and refill code then runs on many lanes at once
         // instead of on one or two lanes nearly every trip.
-        bool finish = pending;
-        const uint32_t refill_batch = W.refill_batch ? W.refill_batch : kRefillBatch;
-        if (refill_batch > 1u) {
-            // both votes are taken by every lane (never inside a short-circuited expression)
-            const unsigned pb = __ballot_sync(FULL, pending);
-            const bool any_active = __any_sync(FULL, active);
-            finish = pending && (uint32_t(__popc(pb)) >= refill_batch || !any_active);
-        }
-        if (finish) {
-            pending = false;
+        const unsigned marching = __ballot_sync(FULL, active), waiting = left & ~marching;
+        if (uint32_t(__popc(waiting)) >= refill_batch || marching == 0u) need = waiting;
+        if ((need >> lane) & 1u) {
             if (W.profile) {
                 atomicAdd(&s_prof[job.shadow ? 2 : (job.bounce == 0u ? 0 : 1)], c_job_orbit);
                 if (m.refine) atomicAdd(&s_prof[3], uint32_t(m.refine));
