@@ -637,6 +637,7 @@ __device__ __forceinline__ void bulb8_step_normal(Orbit<float> &o, float rho2, b
     o.y = __fmaf_rn(a8, __fmul_rn(u4_twice, v4), o.cy);
     o.z = __fmaf_rn(a4_twice, b4, o.cz);
 }
+__device__ __forceinline__ float rho_squared(const Orbit<float> &o) { return __fmaf_rn(o.y, o.y, __fmul_rn(o.x, o.x)); }
 __device__ __forceinline__ float sum_squares(float x, float y, float z) { return __fmaf_rn(z, z, __fmaf_rn(x, x, __fmul_rn(y, y))); }
 
 // One FP32 iteration: step, added constant, squared radius.  o.r is the radius
@@ -645,7 +646,7 @@ template <int KIND>
 __device__ __forceinline__ float orbit_iterate(Orbit<float> &o, const DeviceScene &S, int b8) {
     float r2;
     if (KIND == KIND_BULB8) {
-        const float rho2 = __fmaf_rn(o.y, o.y, __fmul_rn(o.x, o.x));
+        const float rho2 = rho_squared(o);
         if (rho2 >= kSmallestNormal) {
             bulb8_step_normal(o, rho2, b8 == B8_RSQRT);
         } else {
@@ -696,12 +697,26 @@ __device__ __forceinline__ OrbitResult<float> orbit_eval_f32(const DeviceScene &
     if (KIND == KIND_BULB8) o.r = s_sqrt(sum_squares(px, py, pz));
     while (true) {
         bool inside = true;
-        while (inside && o.i < max_iter) {
-            r2 = orbit_iterate<KIND>(o, S, b8);
-            if (KIND == KIND_BULB8) {
+        if (KIND == KIND_BULB8) {
+            // The steps with rho^2 normal; the radius of a step whose square is denormal comes out as 0, which the next
+            // step's r^7 is either way.
+            float rho2 = rho_squared(o);
+            while (inside && rho2 >= kSmallestNormal && o.i < max_iter) {
+                bulb8_step_normal(o, rho2, b8 == B8_RSQRT);
+                ++o.i;
+                o.r = sqrt_normal(sum_squares(o.x, o.y, o.z));
+                inside = o.r <= bailout;
+                rho2 = rho_squared(o);
+            }
+            if (inside && o.i < max_iter) {
+                r2 = orbit_iterate<KIND>(o, S, b8);
                 o.r = s_sqrt(r2);
                 inside = o.r <= bailout;
-            } else {
+                if (inside) continue;
+            }
+        } else {
+            while (inside && o.i < max_iter) {
+                r2 = orbit_iterate<KIND>(o, S, b8);
                 inside = r2 <= S.inside_r2;
             }
         }
@@ -751,9 +766,12 @@ __device__ __forceinline__ OrbitResult<T> ext_field(const DeviceScene &S, T x, T
     if (S.sdf_id == FPT_SDF_MANDELBULBER) {
         float ws = fmaxf(S.set_values[0], 1.0f);
         global_point(S, x, y, z);
-        T inv = T(1.0f / ws);
+        if constexpr (std::is_same<T, float>::value && (KIND == KIND_BULB8 || KIND == KIND_BOX)) {
+            // A world scale of 1, the default, changes nothing: no divisions (20 instructions of an evaluation).
+            if ((KIND == KIND_BOX || b8 != B8_TEMPLATE) && ws == 1.0f)
+                return orbit_eval<KIND, T>(S, x, z, y, ext_iterations(S) * max(mult, 1), ext_bailout(S), b8);
+        }
         OrbitResult<T> o = orbit_eval<KIND, T>(S, x / T(ws), z / T(ws), y / T(ws), ext_iterations(S) * max(mult, 1), ext_bailout(S), b8);
-        (void)inv;
         o.d = o.d * T(ws);
         return o;
     }

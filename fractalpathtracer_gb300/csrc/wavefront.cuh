@@ -32,11 +32,15 @@ namespace fpt {
 // box; the march classifies it as a miss without evaluating.  PF_KNOWN_D:
 // the skip pass handed the ray over with the exact distance at its position
 // in grad.w, so the march does not evaluate it again.
+// PF_MISS: the path ended in the environment along dir; finalize_kernel adds
+// its light (the march kernel evaluated the sky on the few lanes of a finish
+// group that had missed: Menger 720p 16 spp 14.8 -> 14.4 ms, Mandelbox 1080p
+// 4 spp 12.4 -> 11.9 ms).
 // PF_FP64: the camera ray's hit came from the FP64 continuation; its FP64
 // distance from the camera is grad.w + shadow.w (high and low floats).
 enum PathFlags : uint32_t {
     PF_DONE = 1u << 8, PF_INVISIBLE = 1u << 9, PF_VALID = 1u << 10, PF_ESCAPED = 1u << 11, PF_KNOWN_D = 1u << 12,
-    PF_FP64 = 1u << 13
+    PF_FP64 = 1u << 13, PF_MISS = 1u << 14
 };
 
 struct alignas(16) PathRec {
@@ -388,8 +392,9 @@ struct MarchJob {
 // Resident blocks per SM that the register allocation aims at: the Menger fold's
 // short steps are worth more warps (720p 16 spp: 7 blocks 15.6 ms, 8 15.2, 9
 // 14.8, 10 15.1), the others are not (Mandelbulb 1080p 16 spp 28.9 at 7 to 9,
-// Mandelbox 1080p 4 spp 12.4, 12.5, 13.0).
-template <int KIND> constexpr int kMarchBlocks = KIND == KIND_MENGER ? 9 : 7;
+// Mandelbox 1080p 4 spp 12.4, 12.5, 13.0); the power-8 Mandelbulb's kernel, with
+// 64 registers at 8 blocks, loses the eighth at 68 (26.5 against 26.9 ms).
+template <int KIND> constexpr int kMarchBlocks = KIND == KIND_MENGER ? 9 : (KIND == KIND_BULB8 ? 8 : 7);
 // FP64: the camera-ray pass of a deep-zoom scene (FptCudaSceneExt.fp64_bisection,
 // a pinhole camera): a camera ray whose FP32 march stopped because a step no
 // longer moved its position (shaders/Shaders.metal:3726, 3739-3746) continues
@@ -517,7 +522,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
         if (active) {
             const Eval ev = have_d ? Eval{known_d, 0.0f, 0, 0} : scene_eval<KIND>(S, m.pos, EV_MAP, KIND == KIND_BULB8 ? B8_RSQRT : B8_TEMPLATE);
             const float d = ev.d;
-            c_job_orbit += uint32_t(ev.iters);
+            if (W.profile) c_job_orbit += uint32_t(ev.iters);
             have_d = false;
             active = march_update(m, S, d, probe);
             if (active && W.box_on && dot(m.pos - box_origin, m.dir) > box_exit) {
@@ -573,12 +578,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
                 bool hit = !(travel2 > far * far);
                 if (job.bounce == 0u && travel2 > maxd * maxd) R.dir.w = 1.0f;
                 if (!hit) {
-                    float4 dir = R.dir;
-                    float3 env = environment(mk3(dir.x, dir.y, dir.z), S);
-                    float4 col = R.color, li = R.light;
-                    if (S.brdf == FPT_CUDA_BRDF_LAMBERT_GGX) env = env * mk3(col.x, col.y, col.z);
-                    R.light = make_float4(li.x + env.x, li.y + env.y, li.z + env.z, li.w);
-                    R.color.w = bitsf(fbits(col.w) | PF_DONE);
+                    R.color.w = bitsf(fbits(R.color.w) | PF_DONE | PF_MISS);
                     c_paths += 1;
                 } else {
                     R.pos = make_float4(m.pos.x, m.pos.y, m.pos.z, R.pos.w);
@@ -903,7 +903,13 @@ __global__ void __launch_bounds__(256) finalize_kernel(WaveParams W) {
     const DeviceScene &S = BATCH ? W.scenes[state >> 16] : c_scene;
     float3 col = mk3(0.0f);
     if (!(state & PF_INVISIBLE)) {
-        float3 light = mk3(R.light.x + R.shadow.x, R.light.y + R.shadow.y, R.light.z + R.shadow.z);
+        float3 light = mk3(R.light.x, R.light.y, R.light.z);
+        if (state & PF_MISS) {
+            float3 env = environment(mk3(R.dir.x, R.dir.y, R.dir.z), S);
+            if (S.brdf == FPT_CUDA_BRDF_LAMBERT_GGX) env = env * mk3(R.color.x, R.color.y, R.color.z);
+            light = light + env;
+        }
+        light = light + mk3(R.shadow.x, R.shadow.y, R.shadow.z);
         col = S.brdf == FPT_CUDA_BRDF_LAMBERT_GGX ? light : light * mk3(R.color.x, R.color.y, R.color.z);
         if (S.world[6] == 1.0f) col = mix3(col, mk3(R.grad.x, R.grad.y, R.grad.z), R.dir.w);
         col = min3(col, mk3(8.0f));

@@ -151,3 +151,21 @@ def test_mandelbulb8_step_edges(native, iterations, bailout):
     r[flat, 0] = _bulb8_f32(p[flat], iterations, bailout)
     _gate(g[:, 0], r[:, 0], outliers=5e-3)
     assert np.mean(g[:, 3] == r[:, 3]) > 0.995
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.5])
+@pytest.mark.parametrize("box", [False, True])
+def test_world_scale(native, box, scale):
+    """The field's world scale: 1, where nothing is divided, and another."""
+    if box:
+        b = scenes.mandelbox_path(8, 8, 1)
+        cfg, ext, reach = b.cfg, b.ext, 4.0
+    else:
+        cfg, ext = scenes.mandelbulb_primary(8, 8)
+        reach = 1.5
+    cfg.set_values[0] = scale
+    p = pts(1 << 13, -reach * scale, reach * scale, seed=17)
+    g = native.sample_distance(cfg, ext, p)
+    r = oracle.sample_distance(cfg, ext, p, fp64=True)
+    _gate(g[:, 0], r[:, 0])
+    assert np.mean(g[:, 3] == r[:, 3]) > 0.995
