@@ -212,15 +212,20 @@ __device__ __forceinline__ Hit trace(const Grid &g, float3 o, float3 d, uint32_t
 // One loop iteration per visited cell for every lane, so a warp's lanes stay
 // in step (per-lane brick caching and per-lane inner loops over empty bricks
 // were measured slower: whichever lane enters a new brick or leaves an empty
-// one makes the whole warp run that code on most trips).  Per cell: the
-// brick-table word (shift arithmetic, read-only cache), for an occupied brick
-// one mask word, and the advance without the entry-normal writes -- the face
-// normal is rebuilt at the hit from the axis crossed last.  Cells, entry
-// distance, normal and step count of a hit equal trace()'s.  (trace()'s limit
-// of 3 res + 3 steps is never reached: every step leaves a cell for good, and
-// crossing times stay finite.)
-// Bound by issued instructions (ALU pipe 84% before): 1080p primary and shadow rays
-// through the 1024^3 Mandelbox, whose surface fills an eighth of the grid, 2.37 -> 1.42 ms.
+// one makes the whole warp run that code on most trips).  Neither loop returns
+// from its inside: lanes that leave the first loop at different cells then meet
+// after it.  With returns in the loops they did not, and the lanes of a warp
+// walked the box one group after the other.  Per cell: the brick-table word
+// (shift arithmetic, read-only cache), for an occupied brick one mask word, and
+// the advance without the entry-normal writes -- the face normal is rebuilt at
+// the hit from the axis crossed last.  Cells, entry distance, normal and step
+// count of a hit equal trace()'s.  (trace()'s limit of 3 res + 3 steps is never
+// reached: every step leaves a cell for good, and crossing times stay finite.)
+// Bound by issued instructions at 1080p (ALU pipe 84% before the box) and by one
+// warp's chain of cells in small frames.  Whole calls, every cell looked up /
+// box with returns in its loops / this one: 1080p primary and shadow rays
+// through the 1024^3 Mandelbox, whose surface fills an eighth of the grid,
+// 4.68 / 2.83 / 2.07 ms; 64 x 48 rays through 128^3 cells 129 / 344 / 88 us.
 struct AxisPlan {
     float in, out;   // crossing times into and out of the occupied box (estimates), in = -kInfF when inside
     float steps;     // crossings to the way out
@@ -295,51 +300,49 @@ __device__ __forceinline__ Hit trace_bricks(const Grid &g, float3 o, float3 d) {
               end_z = end_cell(step.z, g.occ_lo[2], g.occ_hi[2]);
     int last_axis = -1;   // axis crossed by the last advance (-1: none yet, the normal is the box entry face)
     uint32_t s = 0;
-    // the next crossing: entry time, axes whose boundary it is, cell and crossing times; false when the time cannot advance
+    // The next crossing: entry time, axes whose boundary it is, cell and crossing times.  False when the ray ends: the
+    // time cannot advance, the box is left, or the grid is.
     auto advance_cell = [&]() {
         const float bt = fminf(next_t.x, fminf(next_t.y, next_t.z));
         const bool cx = next_t.x == bt, cy = next_t.y == bt, cz = next_t.z == bt;
-        float ne = bt;
-        if (!(ne > entry_t)) {
-            ne = next_positive_float(entry_t);
-            if (!isfinite(ne) || !(ne > entry_t)) return false;
-        }
+        const float ne = bt > entry_t ? bt : next_positive_float(entry_t);
+        const bool moved = ne > entry_t;
         entry_t = ne;
         last_axis = cx ? 0 : (cy ? 1 : 2);
         if (cx) { cell.x += step.x; next_t.x = next_t.x + delta_t.x; }
         if (cy) { cell.y += step.y; next_t.y = next_t.y + delta_t.y; }
         if (cz) { cell.z += step.z; next_t.z = next_t.z + delta_t.z; }
         ++s;
-        return true;
+        const bool left_box = cell.x == end_x || cell.y == end_y || cell.z == end_z;
+        return moved && !left_box && entry_t <= far_t;
     };
-    auto left_box = [&]() { return cell.x == end_x || cell.y == end_y || cell.z == end_z; };
-    while (outside && entry_t <= far_t) {
-        if (!advance_cell() || left_box()) return h;
+    bool on = entry_t <= far_t;
+    while (outside && on) {
+        on = advance_cell();
         outside = before_box(cell.x, step.x, g.occ_lo[0], g.occ_hi[0]) || before_box(cell.y, step.y, g.occ_lo[1], g.occ_hi[1]) ||
                   before_box(cell.z, step.z, g.occ_lo[2], g.occ_hi[2]);
     }
     const uint32_t bg = g.brick_grid;
     const unsigned long long *mask = reinterpret_cast<const unsigned long long *>(g.mask);
-    while (entry_t <= far_t) {
+    while (on) {
         const uint32_t x = uint32_t(cell.x), y = uint32_t(cell.y), z = uint32_t(cell.z);
         const uint32_t page = __ldg(g.table + (x >> 3) + ((y >> 3) + (z >> 3) * bg) * bg);
-        if (page != 0u && ((__ldg(mask + size_t(page - 1u) * 8u + (z & 7u)) >> ((x & 7u) + 8u * (y & 7u))) & 1ull)) {
-            h.hit = true;
-            h.t = entry_t;
-            h.exit_t = fminf(next_t.x, fminf(next_t.y, next_t.z));
-            h.cell = cell;
-            if (last_axis >= 0) {
-                const int st = last_axis == 0 ? step.x : (last_axis == 1 ? step.y : step.z);
-                const float nv = st > 0 ? -1.0f : 1.0f;
-                h.normal = make_float3(last_axis == 0 ? nv : 0.0f, last_axis == 1 ? nv : 0.0f, last_axis == 2 ? nv : 0.0f);
-            } else {
-                h.normal = en;
-            }
-            h.steps = s + 1;
-            return h;
-        }
-        if (!advance_cell() || left_box()) return h;
+        if (page != 0u && ((__ldg(mask + size_t(page - 1u) * 8u + (z & 7u)) >> ((x & 7u) + 8u * (y & 7u))) & 1ull)) break;
+        on = advance_cell();
     }
+    if (!on) return h;
+    h.hit = true;
+    h.t = entry_t;
+    h.exit_t = fminf(next_t.x, fminf(next_t.y, next_t.z));
+    h.cell = cell;
+    if (last_axis >= 0) {
+        const int st = last_axis == 0 ? step.x : (last_axis == 1 ? step.y : step.z);
+        const float nv = st > 0 ? -1.0f : 1.0f;
+        h.normal = make_float3(last_axis == 0 ? nv : 0.0f, last_axis == 1 ? nv : 0.0f, last_axis == 2 ? nv : 0.0f);
+    } else {
+        h.normal = en;
+    }
+    h.steps = s + 1;
     return h;
 }
 
