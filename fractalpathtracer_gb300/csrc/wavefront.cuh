@@ -11,7 +11,7 @@
 //                   finished takes the next job together with the warp's
 //                   other finished lanes (per-lane regeneration in groups, one
 //                   warp-aggregated atomic per refill); hits go to the shade
-//                   queue, misses add the environment
+//                   queue, misses end the path (finalize_kernel adds the environment)
 //   shade_kernel    material, normal, sun shadow ray, scatter and Russian
 //                   roulette of every hit; continuing paths go back to the
 //                   march queue
@@ -395,6 +395,13 @@ struct MarchJob {
 // Mandelbox 1080p 4 spp 12.4, 12.5, 13.0); the power-8 Mandelbulb's kernel, with
 // 64 registers at 8 blocks, loses the eighth at 68 (26.5 against 26.9 ms).
 template <int KIND> constexpr int kMarchBlocks = KIND == KIND_MENGER ? 9 : (KIND == KIND_BULB8 ? 8 : 7);
+// One vote per trip of the march loop tells who marches, who waits and who is
+// refilled.  Three formulas also vote before the refill and before the
+// evaluation: without those votes their lanes do not stay together (7 spp, 4
+// bounces at 140 x 137, one vote -> three: power-7.3 Mandelbulb 5.76 -> 4.90 ms,
+// hybrid 4.01 -> 3.85, Mandelbox 3.70 -> 3.50; the others lose by them: power-8
+// at 960 x 540 3.79 -> 3.85, Menger 3.03 -> 3.13, 64-scene batch 67.7 -> 69.0).
+template <int KIND> constexpr bool kOneVote = KIND != KIND_BULB && KIND != KIND_HYBRID && KIND != KIND_BOX;
 // FP64: the camera-ray pass of a deep-zoom scene (FptCudaSceneExt.fp64_bisection,
 // a pinhole camera): a camera ray whose FP32 march stopped because a step no
 // longer moved its position (shaders/Shaders.metal:3726, 3739-3746) continues
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
     // The warp's lanes that still take rays, and those of them to refill.  A
     // lane of `left` either marches or waits with a finished ray, so one vote per
     // trip (who marches) tells everything else.
-    unsigned left = FULL, need = FULL;
+    unsigned left = FULL, need = FULL, marching = 0u;
     const uint32_t refill_batch = W.refill_batch ? W.refill_batch : kRefillBatch;
     uint32_t c_primary = 0, c_secondary = 0, c_shadow = 0, c_paths = 0;
     // Profile counters kept off the registers of the march: orbit iterations of
@@ -438,6 +445,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
     while (true) {
         if (loop_guard(trips, t0, W.counters, W.loop_limit_ns)) break;
         // Refill every lane whose march finished: one atomic per warp.
+        if (!kOneVote<KIND>) need = __ballot_sync(FULL, (need >> lane) & 1u);
         if (need) {
             uint32_t leader = __ffs(need) - 1, base = 0;
             if (lane == leader) base = atomicAdd(&W.counters[C_HEAD], (unsigned)__popc(need));
@@ -513,14 +521,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
                 }
             }
             left = __ballot_sync(FULL, !retired);
+            if (KIND == KIND_MENGER) marching = __ballot_sync(FULL, active);
             need = 0u;
         }
-        if (!left) break;
+        if (kOneVote<KIND> ? left == 0u : !__any_sync(FULL, !retired)) break;
         const DeviceScene &S = *sp;
         TranslucencyProbe<KIND> probe{sp};
         // One distance evaluation for every lane with a march in flight.
         if (active) {
             const Eval ev = have_d ? Eval{known_d, 0.0f, 0, 0} : scene_eval<KIND>(S, m.pos, EV_MAP, KIND == KIND_BULB8 ? B8_RSQRT : B8_TEMPLATE);
+            if (KIND == KIND_MENGER) __syncwarp(marching);   // together again after the fold (960 x 540 3.03 -> 2.99 ms)
             const float d = ev.d;
             if (W.profile) c_job_orbit += uint32_t(ev.iters);
             have_d = false;
@@ -536,7 +546,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) march_kernel(WaveParams W, int cu
         // trip) together once `refill_batch` of them wait or nothing else runs:
         // the divergent finish and refill code then runs on many lanes at once
         // instead of on one or two lanes nearly every trip.
-        const unsigned marching = __ballot_sync(FULL, active), waiting = left & ~marching;
+        marching = __ballot_sync(FULL, active);
+        const unsigned waiting = left & ~marching;
         if (uint32_t(__popc(waiting)) >= refill_batch || marching == 0u) need = waiting;
         if ((need >> lane) & 1u) {
             if (W.profile) {

@@ -96,3 +96,21 @@ def test_formula_groups_equal_scene_alone(native, kinds):
     for k, b in enumerate(bundles):
         alone, alone_img, _ = nx.render_batch([b], linear=True, rgba=True)
         assert np.array_equal(lin[k], alone[0]) and np.array_equal(img[k], alone_img[0]), (k, kinds[k])
+
+
+@pytest.mark.parametrize("kind", ["bulb8", "bulb", "box", "menger", "hybrid"])
+@pytest.mark.parametrize("width,height", [(1, 1), (31, 1), (33, 3), (70, 41)])
+def test_refill_groups_do_not_change_images(native, kind, width, height):
+    """Frames of less than a warp's rays, of a ragged last warp and of many refills: how many finished lanes are refilled
+    together and how many warps share the rays changes which lane marches a ray, not the image."""
+    b = _of_kind(kind, 3, width, height, 3)
+    want, want_img, _ = native.cuda_render(b.cfg, b.ext)
+    try:
+        for refill, blocks in ((1, 0), (32, 0), (5, 1)):
+            nx.set_march_schedule(0, refill)
+            nx.set_launch_shape(0, blocks)
+            lin, img, _ = native.cuda_render(b.cfg, b.ext)
+            assert np.array_equal(lin, want) and np.array_equal(img, want_img), (refill, blocks)
+    finally:
+        nx.set_march_schedule(0, 0)
+        nx.set_launch_shape(0, 0)
