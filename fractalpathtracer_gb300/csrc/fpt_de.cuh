@@ -580,7 +580,7 @@ __device__ __forceinline__ float rsqrt_normal(float a) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
-constexpr float kSmallestNormal = 1.17549435e-38f;
+constexpr float kSmallestNormal = 1.17549435e-38f, kLargestFloat = 3.40282347e38f;
 // Two floats in one register pair: the packed operations of this
 // architecture round each half as the scalar operation does.
 using float_pair = unsigned long long;
@@ -695,6 +695,7 @@ __device__ __forceinline__ OrbitResult<float> orbit_eval_f32(const DeviceScene &
     orbit_start(o, px, py, pz);
     float r2 = px * px + py * py + pz * pz;
     if (KIND == KIND_BULB8) o.r = s_sqrt(sum_squares(px, py, pz));
+    const float limit = fminf(bailout, kLargestFloat);   // an infinite radius ends the loop, whatever the bailout radius
     while (true) {
         bool inside = true;
         if (KIND == KIND_BULB8) {
@@ -705,13 +706,13 @@ __device__ __forceinline__ OrbitResult<float> orbit_eval_f32(const DeviceScene &
                 bulb8_step_normal(o, rho2, b8 == B8_RSQRT);
                 ++o.i;
                 o.r = sqrt_normal(sum_squares(o.x, o.y, o.z));
-                inside = o.r <= bailout;
+                inside = o.r <= limit;
                 rho2 = rho_squared(o);
             }
             if (inside && o.i < max_iter) {
                 r2 = orbit_iterate<KIND>(o, S, b8);
                 o.r = s_sqrt(r2);
-                inside = o.r <= bailout;
+                inside = o.r <= limit;
                 if (inside) continue;
             }
         } else {

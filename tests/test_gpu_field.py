@@ -169,3 +169,27 @@ def test_world_scale(native, box, scale):
     r = oracle.sample_distance(cfg, ext, p, fp64=True)
     _gate(g[:, 0], r[:, 0])
     assert np.mean(g[:, 3] == r[:, 3]) > 0.995
+
+
+LARGEST = float(np.finfo(np.float32).max)
+
+
+@pytest.mark.parametrize("route", ["bailout", "set_values"])
+@pytest.mark.parametrize("iterations", [1, 2, 3, 8, 40])
+def test_mandelbulb8_without_bailout(native, iterations, route):
+    """Power-8 orbits that end where FP32 overflows: an infinite bailout radius rolls the last step back like the largest
+    finite one does, bit for bit.  The FP32 oracle is the reference (FP64 overflows some iterations later)."""
+    p = pts(4096, -1.4, 1.4, seed=3)
+    p[:512, :3] *= np.float32(100.0)     # over at the first or second step
+    out = []
+    for bailout in (np.inf, LARGEST):
+        cfg, ext = scenes.mandelbulb_primary(8, 8)
+        ext.iterations = iterations
+        ext.bailout = bailout if route == "bailout" else 0.0
+        cfg.set_values[2] = bailout
+        out.append(native.sample_distance(cfg, ext, p))
+        r = oracle.sample_distance(cfg, ext, p, fp64=False)
+    assert np.isfinite(out[0]).all(axis=0)[[0, 1, 3]].all()   # the derivative of a rolled-back step may overflow
+    assert np.array_equal(out[0], out[1], equal_nan=True)
+    _gate(out[0][:, 0], r[:, 0], outliers=5e-3)
+    assert np.mean(out[0][:, 3] == r[:, 3]) > 0.995

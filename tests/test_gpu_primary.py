@@ -67,3 +67,25 @@ def test_reference_scene_primary_matches_oracle(native):
     assert agree >= 0.98
     assert both.sum() > 100
     assert np.percentile(derr, 95) <= 1e-3
+
+
+@pytest.mark.parametrize("route", ["bailout", "set_values"])
+def test_mandelbulb_without_bailout(native, route):
+    """An infinite bailout radius: hits of the FP32 oracle, and bit for bit those (and the path-traced frame) of the
+    largest finite radius."""
+    hits, frames = [], []
+    for bailout in (np.inf, float(np.finfo(np.float32).max)):
+        cfg, ext = scenes.mandelbulb_primary(160, 120)
+        b = scenes.mandelbulb_path(96, 54, 2)
+        for c, e in ((cfg, ext), (b.cfg, b.ext)):
+            e.bailout = bailout if route == "bailout" else 0.0
+            c.set_values[2] = bailout
+        hits.append(native.trace_primary(cfg, ext)[0])
+        frames.append(native.cuda_render(b.cfg, b.ext)[0])
+        ref = oracle.trace_primary(cfg, ext, fp64=False)
+    assert hits[0].tobytes() == hits[1].tobytes()
+    assert np.array_equal(frames[0], frames[1], equal_nan=True)
+    agree, derr, _, both = _compare(hits[0], ref)
+    assert both.sum() > 2500
+    assert agree >= 0.995, agree
+    assert np.percentile(derr, 99) <= 5e-5, np.percentile(derr, 99)
