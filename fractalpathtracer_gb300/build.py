@@ -47,6 +47,7 @@ def _units():
     units.append(("batch.cu", "batch.o", fast))
     units.append(("bridge.cu", "bridge.o", []))
     units.append(("image_io.cpp", "image_io.o", []))
+    units.append(("host_pages.cpp", "host_pages.o", []))
     missing = sorted({u[0] for u in units if not os.path.exists(os.path.join(CSRC, u[0]))})
     if missing:
         raise RuntimeError(f"listed sources are missing from {CSRC}: {', '.join(missing)}")

@@ -18,13 +18,7 @@
 #include <new>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
-
-#ifdef __linux__
-#include <sys/mman.h>
-#include <unistd.h>
-#endif
 
 #include "fpt_kernels.h"
 #include "fpt_scene.h"
@@ -140,46 +134,6 @@ bool check(cudaError_t e, const char *what, char *error, size_t error_len) {
     if (e == cudaSuccess) return true;
     set_error(error, error_len, "%s failed: %s", what, cudaGetErrorString(e));
     return false;
-}
-
-// A result array that the caller has just allocated has no pages yet.  The copy
-// from the device then takes a fault per page: 1 ms for the 41 MB of a 1080p
-// frame, and up to 35 ms where the GPU takes the faults itself; into populated
-// pages the copy takes 0.3 ms.  Between the launch of the kernels and the
-// wait for them the host is idle, so the pages are populated there
-// (MADV_POPULATE_WRITE: no byte changes, pages that are there are left alone,
-// and on memory or kernels that do not know it the call fails and the copy
-// faults as before).  Clearing pages is bound by one core's 20 GB/s: arrays
-// above 4 MB are shared between up to four threads.
-void populate_pages(std::initializer_list<HostRange> ranges) {
-#ifdef __linux__
-    constexpr int kPopulateWrite = 23;   // MADV_POPULATE_WRITE (Linux 5.14)
-    constexpr size_t kPerThread = size_t(4) << 20;
-    const size_t page = size_t(sysconf(_SC_PAGESIZE));
-    for (const HostRange &r : ranges) {
-        if (!r.data || r.bytes == 0) continue;
-        const uintptr_t begin = (reinterpret_cast<uintptr_t>(r.data) + page - 1) / page * page;
-        const uintptr_t end = (reinterpret_cast<uintptr_t>(r.data) + r.bytes) / page * page;
-        if (end <= begin) continue;
-        const size_t pages = (end - begin) / page;
-        const size_t parts = std::min<size_t>(4, std::max<size_t>(1, (end - begin) / kPerThread));
-        auto part = [=](size_t k) {
-            const uintptr_t a = begin + pages * k / parts * page, b = begin + pages * (k + 1) / parts * page;
-            (void)madvise(reinterpret_cast<void *>(a), b - a, kPopulateWrite);
-        };
-        std::thread helpers[3];
-        size_t started = 0;
-        try {
-            for (; started + 1 < parts; ++started) helpers[started] = std::thread(part, started + 1);
-        } catch (...) {   // no thread to be had: the rest is done here
-        }
-        part(0);
-        for (size_t k = started + 1; k < parts; ++k) part(k);
-        for (size_t k = 0; k < started; ++k) helpers[k].join();
-    }
-#else
-    (void)ranges;
-#endif
 }
 
 // ------------------------------------------------------------------ scene compilation

@@ -3,10 +3,10 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <initializer_list>
 #include <mutex>
 
 #include "fpt_scene.h"
+#include "host_pages.h"
 
 namespace fpt {
 
@@ -49,13 +49,6 @@ void set_error(char *error, size_t error_len, const char *fmt, ...);
 bool ensure_device(char *error, size_t error_len);
 bool ensure_buffer(void **ptr, size_t *cap, size_t need, char *error, size_t error_len);
 bool check(cudaError_t e, const char *what, char *error, size_t error_len);
-// Gives the pages of result arrays that the caller has only reserved so far
-// their memory, while the GPU works on the results.
-struct HostRange {
-    void *data;
-    size_t bytes;
-};
-void populate_pages(std::initializer_list<HostRange> ranges);
 bool compile_scene(const FptRenderConfig &c, const FptCudaSceneExt *ext, DeviceScene &S, char *error, size_t error_len);
 bool hydrate_hdri(FptRenderConfig &config, char *error, size_t error_len);
 bool upload_scene(DeviceScene &S, const FptCudaSceneExt *ext, char *error, size_t error_len);
