@@ -29,6 +29,7 @@
 #include <mutex>
 #include <vector>
 
+#include "batch_branches.h"
 #include "bridge_internal.h"
 #include "render_impl.cuh"
 
@@ -73,9 +74,7 @@ struct BatchState {
     float4 *sample_rgb = nullptr; size_t cap_sample = 0;
     uchar4 *rgba = nullptr; size_t cap_rgba = 0;
     uint32_t *counters = nullptr; size_t cap_counters = 0;   // kCounterStride words per formula group
-    // Branches of the pass graph (formula groups beyond the first) and the events that fork and join them.
-    cudaStream_t branch[kMaxGroups] = {};
-    cudaEvent_t fork = nullptr, join[kMaxGroups] = {};
+    BranchSet<kMaxGroups> branches;   // of the pass graph: one formula group each
 };
 BatchState &bstate() {
     static BatchState b;
@@ -212,13 +211,7 @@ bool upload_plan(const BatchPlan &P, uint32_t wave_paths, char *error, size_t er
         !ensure_buffer(&c.wave, &c.cap_wave, scratch, error, error_len) ||
         !ensure_buffer((void **)&B.counters, &B.cap_counters, kMaxGroups * kCounterStride * sizeof(uint32_t), error, error_len))
         return false;
-    if (!B.fork) {
-        bool ok = check(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming), "batch events", error, error_len);
-        for (int k = 1; ok && k < kMaxGroups; ++k)
-            ok = check(cudaEventCreateWithFlags(&B.join[k], cudaEventDisableTiming), "batch events", error, error_len) &&
-                 check(cudaStreamCreateWithFlags(&B.branch[k], cudaStreamNonBlocking), "batch branches", error, error_len);
-        if (!ok) return false;
-    }
+    if (!check(B.branches.create(), "batch branches", error, error_len)) return false;
     std::vector<uint32_t> tables(2 * (n + 1) + 1, 0u);
     std::copy(P.work_base.begin(), P.work_base.end(), tables.begin());
     std::copy(P.pixel_base.begin(), P.pixel_base.end(), tables.begin() + (n + 1));
@@ -293,25 +286,27 @@ uint32_t launch_group(const BatchPlan &P, size_t group, char *scratch, const Mar
 }
 
 // Launches one pass of the batch, forked from and joined into `st` (captured
-// into the graph).  Returns the number of kernel launches.
-uint32_t launch_pass(const BatchPlan &P, const MarchVariant &V, uint32_t wave_paths, uint32_t refill, cudaStream_t st) {
+// into the graph).  `launches`: the number of kernel launches.
+cudaError_t launch_pass(const BatchPlan &P, const MarchVariant &V, uint32_t wave_paths, uint32_t refill, cudaStream_t st,
+                        uint32_t &launches) {
     BatchState &B = bstate();
     const size_t n = P.scenes.size();
-    uint32_t launches = 0;
     char *scratch = static_cast<char *>(ctx().wave);
-    cudaEventRecord(B.fork, st);
-    for (size_t k = 0; k < P.groups.size(); ++k) {
-        const cudaStream_t on = k == 0 ? st : B.branch[k];
-        if (k > 0) cudaStreamWaitEvent(on, B.fork, 0);
-        launches += launch_group(P, k, scratch, V, wave_paths, refill, on);
+    launches = 0;
+    cudaError_t e = B.branches.begin(st);
+    for (size_t k = 0; k < P.groups.size() && e == cudaSuccess; ++k) {
+        e = B.branches.enter(int(k));
+        if (e != cudaSuccess) break;
+        launches += launch_group(P, k, scratch, V, wave_paths, refill, B.branches.branch(int(k), st));
         scratch += group_scratch(P, P.groups[k], wave_paths);
-        if (k > 0) cudaEventRecord(B.join[k], on);
+        e = B.branches.leave(int(k), st);
     }
-    for (size_t k = 1; k < P.groups.size(); ++k) cudaStreamWaitEvent(st, B.join[k], 0);
+    if (e != cudaSuccess) return e;
     reduce_pass_kernel<<<uint32_t((P.pixels + 255) / 256), 256, 0, st>>>(B.sample_rgb, B.accum, uint32_t(P.pixels),
                                                                         B.tables + 2 * (n + 1));
     advance_pass_kernel<<<1, 32, 0, st>>>(B.tables + 2 * (n + 1));
-    return launches + 2;
+    launches += 2;
+    return cudaSuccess;
 }
 
 // Captures one pass into a graph.
@@ -321,8 +316,12 @@ bool capture_pass(const BatchPlan &P, const MarchVariant &V, uint32_t wave_paths
     Context &c = ctx();
     cudaGraph_t graph = nullptr;
     if (!check(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal), "graph capture", error, error_len)) return false;
-    launches = launch_pass(P, V, wave_paths, refill, c.stream);
+    const cudaError_t forked = launch_pass(P, V, wave_paths, refill, c.stream, launches);
     cudaError_t e = cudaStreamEndCapture(c.stream, &graph);
+    if (!check(forked, "batch branches", error, error_len)) {
+        if (graph) cudaGraphDestroy(graph);
+        return false;
+    }
     if (!check(e, "graph capture", error, error_len)) return false;
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
