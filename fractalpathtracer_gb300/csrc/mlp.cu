@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "bridge_internal.h"
+#include "chain_launch.h"
 #include "fpt_kernels.h"
 #include "fpt_math.cuh"
 #include "mlp.cuh"
@@ -892,31 +893,16 @@ static void set_attributes() {
     done = true;
 }
 
-// Launches a kernel of the training chain; `early`: it may start while the kernel before it ends.
-template <class... P, class... A>
-static void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool early, A... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(unsigned(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = early ? 1u : 0u;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // Forward + backward of one batch: accumulates into A.grad and A.loss, or, with `adam` (its parameters, moments and
-// step), takes the Adam step and accumulates the loss.
+// step), takes the Adam step and accumulates the loss.  The status is that of the first refused launch.
 // `next`: the pass follows the Adam step of another in the stream (its kernels, nothing between).
-static void launch_gradients(const TrainArgs &A, const SumArgs *adam, bool next, cudaStream_t st) {
+static cudaError_t launch_gradients(const TrainArgs &A, const SumArgs *adam, bool next, cudaStream_t st) {
     set_attributes();
+    ChainLaunch chain(st);
     const uint32_t blocks = (A.batch + kRowsPerBlock - 1) / kRowsPerBlock;
     // forward + backward on the network engine of the inference passes (tcgen05 by default)
-    if (ctx().network_engine == FPT_CUDA_NET_MMA_SYNC) train_fwd_bwd_kernel<<<blocks, 32 * kWarpsTrain, train_smem_bytes(), st>>>(A);
-    else launch_chained(train_fwd_bwd_tc_kernel, dim3(blocks), kTrainThreads, train_tc_smem_bytes(), st, next, A);
+    if (ctx().network_engine == FPT_CUDA_NET_MMA_SYNC) chain.launch(train_fwd_bwd_kernel, dim3(blocks), 32 * kWarpsTrain, train_smem_bytes(), false, A);
+    else chain.launch(train_fwd_bwd_tc_kernel, dim3(blocks), kTrainThreads, train_tc_smem_bytes(), next, A);
     WgradArgs G;
     G.h[0] = A.gx;
     for (int l = 1; l < kHidden; ++l) G.h[l] = A.gh[l - 1];
@@ -925,7 +911,7 @@ static void launch_gradients(const TrainArgs &A, const SumArgs *adam, bool next,
     G.chunks = wgrad_chunks(A.batch);
     G.part = A.w_part;
     G.fail = A.fail;
-    launch_chained(wgrad_tc_kernel, dim3(G.chunks, kHidden), kTcRows, wgrad_smem_bytes(), st, true, G);
+    chain.launch(wgrad_tc_kernel, dim3(G.chunks, kHidden), kTcRows, wgrad_smem_bytes(), true, G);
     SumArgs S = adam ? *adam : SumArgs{};
     S.w_part = A.w_part;
     S.out_part = A.out_part;
@@ -933,8 +919,9 @@ static void launch_gradients(const TrainArgs &A, const SumArgs *adam, bool next,
     S.warps = blocks * kWarpsTrain;
     S.grad = A.grad;
     S.loss = A.loss;
-    if (adam) launch_chained(gradient_kernel<true>, dim3(kSumBlocks), kTcRows, 0, st, true, S);
-    else launch_chained(gradient_kernel<false>, dim3(kSumBlocks), kTcRows, 0, st, true, S);
+    if (adam) chain.launch(gradient_kernel<true>, dim3(kSumBlocks), kTcRows, 0, true, S);
+    else chain.launch(gradient_kernel<false>, dim3(kSumBlocks), kTcRows, 0, true, S);
+    return chain.status;
 }
 
 static HostModel *find(uint64_t id) {
@@ -1098,7 +1085,10 @@ int fpt_cuda_mlp_create(const struct FptRenderConfig *config, const struct FptCu
         const float lr0 = mc->lr > 0.0f ? mc->lr : 2e-3f;
         for (uint32_t s = 0; s < mc->steps; ++s) {
             const bool probe = s == 0 || s + 1 == mc->steps;
-            if (probe) cudaMemsetAsync(hm->loss, 0, 4, c.stream);
+            if (probe && !check(cudaMemsetAsync(hm->loss, 0, 4, c.stream), "loss reset", error, error_len)) {
+                mlp::free_model(hm);
+                return 1;
+            }
             mlp::TrainArgs A;
             mlp::fill_train_args(A, *hm, hm->data, hm->n_data, mc->batch, over);
             A.seed = seed;
@@ -1108,7 +1098,11 @@ int fpt_cuda_mlp_create(const struct FptRenderConfig *config, const struct FptCu
             mlp::SumArgs adam{};
             adam.params = hm->params; adam.m = hm->m; adam.v = hm->v; adam.wbf = hm->wbf;
             adam.lr = lr; adam.b1t = b1t; adam.b2t = b2t;
-            mlp::launch_gradients(A, &adam, s > 0, c.stream);
+            if (!check(mlp::launch_gradients(A, &adam, s > 0, c.stream), "training step launch", error, error_len)) {
+                cudaStreamSynchronize(c.stream);   // the steps before it still use the model
+                mlp::free_model(hm);
+                return 1;
+            }
             if (probe) {
                 float l = 0.0f;
                 if (!check(cudaMemcpyAsync(&l, hm->loss, 4, cudaMemcpyDeviceToHost, c.stream), "loss readback", error, error_len) ||
@@ -1257,9 +1251,8 @@ int fpt_cuda_mlp_gradients(uint64_t model, const float *points_xyzw, size_t n, f
               check(cudaMemsetAsync(hm->grad, 0, mlp::kParams * 4, c.stream), "grad reset", error, error_len) &&
               check(cudaMemsetAsync(hm->loss, 0, 4, c.stream), "loss reset", error, error_len);
     if (!ok) return 1;
-    mlp::launch_gradients(A, nullptr, false, c.stream);
     float l = 0.0f;
-    ok = check(cudaGetLastError(), "gradient launch", error, error_len) &&
+    ok = check(mlp::launch_gradients(A, nullptr, false, c.stream), "gradient launch", error, error_len) &&
          check(cudaMemcpyAsync(gradients, hm->grad, mlp::kParams * 4, cudaMemcpyDeviceToHost, c.stream), "gradient readback", error, error_len) &&
          check(cudaMemcpyAsync(&l, hm->loss, 4, cudaMemcpyDeviceToHost, c.stream), "loss readback", error, error_len) &&
          check(cudaMemsetAsync(hm->grad, 0, mlp::kParams * 4, c.stream), "grad reset", error, error_len) &&
