@@ -894,15 +894,14 @@ static void set_attributes() {
 }
 
 // Forward + backward of one batch: accumulates into A.grad and A.loss, or, with `adam` (its parameters, moments and
-// step), takes the Adam step and accumulates the loss.  The status is that of the first refused launch.
-// `next`: the pass follows the Adam step of another in the stream (its kernels, nothing between).
-static cudaError_t launch_gradients(const TrainArgs &A, const SumArgs *adam, bool next, cudaStream_t st) {
+// step), takes the Adam step and accumulates the loss.  Within a pass, and from the Adam step of a pass to the next, the
+// kernels overlap.  The chain's status is that of the first refused launch.
+static void launch_gradients(const TrainArgs &A, const SumArgs *adam, ChainLaunch &chain) {
     set_attributes();
-    ChainLaunch chain(st);
     const uint32_t blocks = (A.batch + kRowsPerBlock - 1) / kRowsPerBlock;
     // forward + backward on the network engine of the inference passes (tcgen05 by default)
     if (ctx().network_engine == FPT_CUDA_NET_MMA_SYNC) chain.launch(train_fwd_bwd_kernel, dim3(blocks), 32 * kWarpsTrain, train_smem_bytes(), false, A);
-    else chain.launch(train_fwd_bwd_tc_kernel, dim3(blocks), kTrainThreads, train_tc_smem_bytes(), next, A);
+    else chain.launch(train_fwd_bwd_tc_kernel, dim3(blocks), kTrainThreads, train_tc_smem_bytes(), true, A);
     WgradArgs G;
     G.h[0] = A.gx;
     for (int l = 1; l < kHidden; ++l) G.h[l] = A.gh[l - 1];
@@ -921,7 +920,6 @@ static cudaError_t launch_gradients(const TrainArgs &A, const SumArgs *adam, boo
     S.loss = A.loss;
     if (adam) chain.launch(gradient_kernel<true>, dim3(kSumBlocks), kTcRows, 0, true, S);
     else chain.launch(gradient_kernel<false>, dim3(kSumBlocks), kTcRows, 0, true, S);
-    return chain.status;
 }
 
 static HostModel *find(uint64_t id) {
@@ -1083,12 +1081,10 @@ int fpt_cuda_mlp_create(const struct FptRenderConfig *config, const struct FptCu
         if (!mlp::ensure_rows(*hm, mc->batch, error, error_len)) { mlp::free_model(hm); return 1; }
         const float over = mc->overestimate_weight > 0.0f ? mc->overestimate_weight : 10.0f;
         const float lr0 = mc->lr > 0.0f ? mc->lr : 2e-3f;
+        ChainLaunch chain(c.stream);
         for (uint32_t s = 0; s < mc->steps; ++s) {
             const bool probe = s == 0 || s + 1 == mc->steps;
-            if (probe && !check(cudaMemsetAsync(hm->loss, 0, 4, c.stream), "loss reset", error, error_len)) {
-                mlp::free_model(hm);
-                return 1;
-            }
+            if (probe) chain.zero(hm->loss, 4);
             mlp::TrainArgs A;
             mlp::fill_train_args(A, *hm, hm->data, hm->n_data, mc->batch, over);
             A.seed = seed;
@@ -1098,15 +1094,16 @@ int fpt_cuda_mlp_create(const struct FptRenderConfig *config, const struct FptCu
             mlp::SumArgs adam{};
             adam.params = hm->params; adam.m = hm->m; adam.v = hm->v; adam.wbf = hm->wbf;
             adam.lr = lr; adam.b1t = b1t; adam.b2t = b2t;
-            if (!check(mlp::launch_gradients(A, &adam, s > 0, c.stream), "training step launch", error, error_len)) {
+            mlp::launch_gradients(A, &adam, chain);
+            float l = 0.0f;
+            if (probe) chain.read(&l, hm->loss, 4);
+            if (!check(chain.status, "training step launch", error, error_len)) {
                 cudaStreamSynchronize(c.stream);   // the steps before it still use the model
                 mlp::free_model(hm);
                 return 1;
             }
             if (probe) {
-                float l = 0.0f;
-                if (!check(cudaMemcpyAsync(&l, hm->loss, 4, cudaMemcpyDeviceToHost, c.stream), "loss readback", error, error_len) ||
-                    !check(cudaStreamSynchronize(c.stream), "training step", error, error_len)) {
+                if (!check(cudaStreamSynchronize(c.stream), "training step", error, error_len)) {
                     mlp::free_model(hm);
                     return 1;
                 }
@@ -1252,7 +1249,9 @@ int fpt_cuda_mlp_gradients(uint64_t model, const float *points_xyzw, size_t n, f
               check(cudaMemsetAsync(hm->loss, 0, 4, c.stream), "loss reset", error, error_len);
     if (!ok) return 1;
     float l = 0.0f;
-    ok = check(mlp::launch_gradients(A, nullptr, false, c.stream), "gradient launch", error, error_len) &&
+    ChainLaunch chain(c.stream);
+    mlp::launch_gradients(A, nullptr, chain);
+    ok = check(chain.status, "gradient launch", error, error_len) &&
          check(cudaMemcpyAsync(gradients, hm->grad, mlp::kParams * 4, cudaMemcpyDeviceToHost, c.stream), "gradient readback", error, error_len) &&
          check(cudaMemcpyAsync(&l, hm->loss, 4, cudaMemcpyDeviceToHost, c.stream), "loss readback", error, error_len) &&
          check(cudaMemsetAsync(hm->grad, 0, mlp::kParams * 4, c.stream), "grad reset", error, error_len) &&

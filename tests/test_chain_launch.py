@@ -61,3 +61,54 @@ def test_launches_pass_their_arguments(lines):
 def test_refused_launch_is_kept_and_ends_the_chain(lines):
     ends = [[int(v) for v in line.split()[1:]] for line in lines if line.startswith("end")]
     assert ends == [[0, 0, 3, 0], [1, 9, 1, 1], [2, 9, 2, 1], [3, 9, 3, 1]]   # 9: invalid configuration
+
+
+GAPS = r"""
+#include <stdio.h>
+#include "chain_launch.h"
+static int refuse = 0;
+static void kernel(int) {}
+extern "C" {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) { printf("%u ", c->numAttrs); return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void *, int v, size_t n, cudaStream_t) {
+    printf("zero%d:%zu ", v, n);
+    return refuse == 1 ? cudaErrorInvalidValue : cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *, const void *, size_t n, cudaMemcpyKind k, cudaStream_t) {
+    printf("read%d:%zu ", int(k), n);
+    return refuse == 2 ? cudaErrorInvalidValue : cudaSuccess;
+}
+}
+int main() {
+    for (refuse = 0; refuse < 3; ++refuse) {
+        float loss = 0.0f;
+        fpt::ChainLaunch chain(nullptr);
+        for (int step = 0; step < 4; ++step) {   // a training of four steps: the loss of the first and the last is read
+            const bool probe = step == 0 || step == 3;
+            if (probe) chain.zero(&loss, 4);
+            chain.launch(kernel, dim3(1), 32, 0, true, 1);
+            chain.launch(kernel, dim3(1), 32, 0, false, 1);
+            chain.launch(kernel, dim3(1), 32, 0, true, 1);
+            if (probe) chain.read(&loss, &loss, 4);
+        }
+        printf("status%d\n", int(chain.status));
+    }
+    return 0;
+}
+"""
+
+
+def test_no_overlap_behind_copies_and_memsets(tmp_path):
+    """A kernel of the chain may start early behind another kernel of it only, and a refused memset or copy ends the chain."""
+    gxx = shutil.which("g++")
+    if gxx is None or not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime_api.h")):
+        pytest.skip("g++ or the CUDA headers are not available")
+    (tmp_path / "main.cpp").write_text(GAPS)
+    exe = str(tmp_path / "gaps")
+    subprocess.run([gxx, "-std=c++17", "-I", os.path.join(ROOT, "fractalpathtracer_gb300", "csrc"), "-I", CUDA_INCLUDE,
+                    str(tmp_path / "main.cpp"), "-o", exe], check=True, capture_output=True, text=True)
+    lines = subprocess.run([exe], check=True, capture_output=True, text=True).stdout.splitlines()
+    assert lines[0] == "zero0:4 0 0 1 read2:4 0 0 1 1 0 1 zero0:4 0 0 1 read2:4 status0"
+    assert lines[1] == "zero0:4 status1"
+    assert lines[2] == "zero0:4 0 0 1 read2:4 status1"
