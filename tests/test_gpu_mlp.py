@@ -155,6 +155,62 @@ def test_training_is_deterministic(native):
     assert np.array_equal(params[0], params[1])
 
 
+def _pcg(v):
+    v = np.asarray(v, np.uint32)
+    state = v * np.uint32(747796405) + np.uint32(2891336453)
+    word = ((state >> ((state >> np.uint32(28)) + np.uint32(4))) ^ state) * np.uint32(277803737)
+    return (word >> np.uint32(22)) ^ word
+
+
+@pytest.mark.parametrize("engine", ENGINES, indirect=True)
+@pytest.mark.parametrize("rows,steps", [(64, 1), (333, 2), (4096 + 77, 3)])
+def test_training_steps_match_adam_on_the_host(native, blank_model, engine, rows, steps):
+    """One to three training steps, ragged batches among them, against Adam in FP32 on the host with the gradients of
+    fpt_cuda_mlp_gradients at the same rows.  A parameter moves by at most about lr a step; the host's separately rounded
+    operations and the few BF16 weights that they flip change a step by less than 1e-5 (0.5% of lr) for nearly all.  The
+    BF16 weights of the trained model are those of its parameters, and the padding columns of W0 stay zero."""
+    cfg, ext = scenes.mandelbulb_primary(8, 8)
+    points, seed, lr0 = 2048, 21, 2e-3
+    mc = nx.mlp_config(*BULB_BOX, points=points, near_fraction=0.0, steps=steps, batch=rows, lr=lr0, seed=seed)
+    h, _ = nx.mlp_create(cfg, ext, mc)
+    try:
+        trained = nx.mlp_get_params(h)
+        probe = _points(1000, 4)
+        predicted = nx.mlp_predict(h, probe)
+    finally:
+        nx.mlp_destroy(h)
+    h, _ = nx.mlp_create(cfg, ext, nx.mlp_config(*BULB_BOX, points=0, steps=0, seed=seed))
+    try:
+        p = nx.mlp_get_params(h)
+    finally:
+        nx.mlp_destroy(h)
+    index = np.arange(points, dtype=np.uint32)
+    hashed = _pcg(np.uint32(seed) ^ _pcg(index))
+    data = np.zeros((points, 4), np.float32)
+    lo, hi = (np.asarray(b, np.float64) for b in BULB_BOX)
+    for k in range(3):
+        data[:, k] = lo[k] + (hi[k] - lo[k]) * ((_pcg(hashed + np.uint32(k)) >> np.uint32(8)) / 16777216.0)
+    data[:, 3] = native.sample_distance(cfg, ext, data)[:, 0]
+    f = np.float32
+    m, v = np.zeros_like(p), np.zeros_like(p)
+    for s in range(steps):
+        nx.mlp_set_params(blank_model, p)
+        pick = _pcg(np.uint32(seed + 7919 * s) ^ _pcg(np.arange(rows, dtype=np.uint32))) % np.uint32(points)
+        g, _ = nx.mlp_gradients(blank_model, data[pick], 10.0)
+        g[:7168].reshape(64, 112)[:, 99:] = 0.0
+        lr = f(max(lr0 * 0.5 * (1.0 + np.cos(np.pi * s / steps)), lr0 * 0.02))
+        m = f(0.9) * m + f(0.1) * g
+        v = f(0.999) * v + f(0.001) * g * g
+        p = p - lr * (m / f(1.0 - 0.9 ** (s + 1))) / (np.sqrt(v / f(1.0 - 0.999 ** (s + 1))) + f(1e-8))
+    off = np.abs(trained - p)
+    print(f"{rows} rows, {steps} steps: max {off.max():.2e} p99.5 {np.percentile(off, 99.5):.2e}")
+    assert np.percentile(off, 99.5) <= 1e-5
+    assert off.max() <= 2 * lr0 * steps
+    assert not trained[:7168].reshape(64, 112)[:, 99:].any()
+    nx.mlp_set_params(blank_model, trained)
+    assert np.array_equal(nx.mlp_predict(blank_model, probe), predicted)
+
+
 @pytest.fixture(scope="module")
 def trained_bulb(native):
     cfg, ext = scenes.mandelbulb_primary(8, 8)
