@@ -797,7 +797,7 @@ struct HostModel {
     __nv_bfloat16 *wbf = nullptr;
     float4 *data = nullptr;
     uint32_t n_data = 0;
-    __nv_bfloat16 *act = nullptr;   // gx | gh[3] | gz[4] | gdz[4]
+    __nv_bfloat16 *act = nullptr;   // gx | gh[3] | gz[4] (mma.sync pass only) | gdz[4]
     float *part = nullptr;          // gradient partials: wgrad_tc_kernel chunks, then train-kernel warps, then the fail word
     uint32_t rows_cap = 0;
     float center[3] = {0, 0, 0}, inv_half[3] = {1, 1, 1}, lo[3] = {-1, -1, -1}, hi[3] = {1, 1, 1}, label_scale = 1.0f;
@@ -824,7 +824,7 @@ static void free_model(HostModel *hm) {
     delete hm;
 }
 
-// Partial sums of a batch of `rows`: [4 layers][chunks][128][64] for the
+// Partial sums of a batch of `rows`: [4 layers][chunks][64 n][128 m] for the
 // weight gradients, [warps][kOutPart] for the output layer and loss, and one
 // word for MMA time-outs.
 static uint32_t wgrad_chunks(uint32_t rows) { return (rows + kWgChunk - 1) / kWgChunk; }

@@ -401,6 +401,10 @@ template <int KIND> constexpr int kMarchBlocks = KIND == KIND_MENGER ? 9 : (KIND
 // bounces at 140 x 137, one vote -> three: power-7.3 Mandelbulb 5.76 -> 4.90 ms,
 // hybrid 4.01 -> 3.85, Mandelbox 3.70 -> 3.50; the others lose by them: power-8
 // at 960 x 540 3.79 -> 3.85, Menger 3.03 -> 3.13, 64-scene batch 67.7 -> 69.0).
+// The Mandelbox, one vote -> three, over its sizes: 64 x 48 4 spp 2.41 -> 2.42,
+// 140 x 137 7 spp 3.54 -> 3.43, 333 x 217 2 spp 2.72 -> 2.65, 640 x 360 4 spp
+// 4.41 -> 4.38, 960 x 540 4 spp 5.61 -> 5.62, 1080p 1 spp 5.71 -> 5.71, 16 spp
+// 38.1 -> 38.4 ms: more at small frames than the large ones lose.
 template <int KIND> constexpr bool kOneVote = KIND != KIND_BULB && KIND != KIND_HYBRID && KIND != KIND_BOX;
 // FP64: the camera-ray pass of a deep-zoom scene (FptCudaSceneExt.fp64_bisection,
 // a pinhole camera): a camera ray whose FP32 march stopped because a step no

@@ -212,3 +212,12 @@ def test_results_into_part_of_an_array(native, width, height, offset):
     assert np.array_equal(got, want) and np.array_equal(got_img, want_img)
     assert not lin[:offset].any() and not lin[offset + n:].any()
     assert (img[:offset] == 7).all() and (img[offset + n:] == 9).all()
+
+
+@pytest.mark.parametrize("iterations,bailout", [(1, 2.0), (2, 50.0), (5, 50.0)])
+def test_mandelbulb_orbit_ends(native, iterations, bailout):
+    """The march kernel's power-8 loop where orbits end at the first iteration, at the last one or far outside
+    (the tolerance of test_mandelbulb_path)."""
+    b = scenes.mandelbulb_path(96, 54, 2)
+    b.ext.iterations, b.ext.bailout = iterations, bailout
+    _check(native, b.cfg, b.ext, mae=3.0, rmse=12.0, ssim=0.9, lf=0.98)
